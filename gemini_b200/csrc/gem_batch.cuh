@@ -122,9 +122,10 @@ __global__ void __launch_bounds__(128) kb_clean_vel_edges(const InstDev* __restr
 // (LU_WPB warp tasks) of an instance; the grid never exceeds the scratch slots, and each
 // resident warp keeps the slot of its (block, warp) for every item it runs.
 template <bool UNIT>
-__global__ void __launch_bounds__(32 * LU_WPB, GEM_LU_MINB) kb_diffusion_lu(const InstDev* __restrict__ inst,
+__global__ void __launch_bounds__(32 * LU_WPB, LU_MINB) kb_diffusion_lu(const InstDev* __restrict__ inst,
                                                               const Item* __restrict__ it, int n, double* lu,
                                                               long long lu_slot) {
+  __shared__ LuTiles tiles[LU_WPB];
   const int warp = threadIdx.x >> 5;
   double* slot = lu + (long long)(blockIdx.x * LU_WPB + warp) * lu_slot;
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(32 * LU_WPB, GEM_LU_MINB) kb_diffusion_lu(cons
     const int ncol = P.G.d.lx2 * P.G.d.lx3;
     const int ntask = ((ncol + 31) / 32) * LSP;
     const int t = q.y * LU_WPB + warp;
-    if (t < ntask) b_diffusion_lu<UNIT>(P, t, slot);
+    if (t < ntask) b_diffusion_lu<UNIT>(P, t, slot, tiles[warp]);
   }
 }
 
@@ -164,7 +165,7 @@ struct gem_batch {
   std::vector<gem_work*> works;
   InstDev* d_inst = nullptr;
   std::vector<BatchLaunch> launches;  // in step order
-  int diff_blocks = LU_MINB_DEFAULT;  // diffusion blocks per SM (each LU_WPB warps)
+  int diff_blocks = LU_MINB;  // diffusion blocks per SM (each LU_WPB warps)
   int per_sm_scale = 100;  // percent of the occupancy-limited persistent grid
   cudaStream_t cap_stream = nullptr;
   cudaGraph_t graph = nullptr;
@@ -457,8 +458,8 @@ int gem_batch_set_param(gem_batch* b, int param, int value) {
     return GEM_OK;
   }
   if (param == GEM_BATCH_DIFF_BLOCKS) {
-    if (value < 1 || value > LU_MINB_DEFAULT)
-      return set_err(GEM_EINVAL, "diffusion blocks per SM %d: 1..%d", value, LU_MINB_DEFAULT);
+    if (value < 1 || value > LU_MINB)
+      return set_err(GEM_EINVAL, "diffusion blocks per SM %d: 1..%d", value, LU_MINB);
     b->diff_blocks = value;
   } else if (param == GEM_BATCH_GRID_PCT) {
     if (value != 0 && (value < 10 || value > 400))

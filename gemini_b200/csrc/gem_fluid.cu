@@ -236,15 +236,15 @@ int lu_warps_per_sm() {
   static int wps = 0;
   if (!wps) {
     int a = 0, b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_diffusion_lu<true>, 32 * LU_WPB, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_diffusion_lu<false>, 32 * LU_WPB, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_diffusion_lu<true, LU_MINB>, 32 * LU_WPB, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_diffusion_lu<false, LU_MINB>, 32 * LU_WPB, 0);
     const int w = std::min(a, b) * LU_WPB;
     wps = std::max(LU_WPB, std::min(w, LU_MAX_WARPS_PER_SM));
   }
   return wps;
 }
 long long lu_slots() { return (long long)num_sms() * lu_warps_per_sm(); }
-long long lu_slot_doubles(int lx1) { return (long long)lx1 * gemd::LU_ROW * 32; }
+long long lu_slot_doubles(int lx1) { return lu_lane_doubles(lx1) * 32; }
 // warp tasks of one grid's diffusion, rounded up to whole blocks
 long long lu_tasks(const Dims& d) {
   const long long ntask = (((long long)d.lx2 * d.lx3 + 31) / 32) * LSP;
@@ -267,16 +267,51 @@ int work_lu(gem_work* w, const gem_grid* g, double** out) {
   return GEM_OK;
 }
 
+// Columns per block of k_diffusion_col, 0 where k_diffusion_lu runs instead.
+// k_diffusion_lu takes about 2 us per x1 row however few columns there are (one thread's
+// chain through four passes) and slows down only beyond 12 warps per SM.  k_diffusion_col
+// takes about 0.5 us per row and round (fit columns per SM in shared memory at a time: the
+// chain of the solving threads) plus 0.006 us per row and column of an SM (forming the rows,
+// whole warps along x1).  The line is where the two meet; measured, us per launch, col / lu:
+// 64x8x6 36 / 120, 96x32x32 79 / 182, 384x24x24 505 / 769, 173x45x37 326 / 403,
+// 128x64x64 470 / 288, 64x96x96 371 / 206.
+size_t luc_bytes(int lx1) { return sizeof(double) * luc_pitch(lx1); }
+int luc_columns(const Dims& d) {
+  constexpr size_t SM_BYTES = 227 * 1024, BLOCK_OVERHEAD = 1024;
+  const long long ncol = (long long)d.lx2 * d.lx3;
+  const long long per_sm = (ncol * LSP + num_sms() - 1) / num_sms();  // (column, species) pairs per SM
+  const long long fit = (long long)(SM_BYTES / luc_bytes(d.lx1));
+  if (fit < 1 || lu_tasks(d) > lu_slots()) return 0;  // the scratch holds every column
+  const long long rounds = (per_sm + fit - 1) / fit;
+  const long long warp_rows = 32LL * ((d.lx1 + 31) / 32);  // rows a column occupies in whole warps
+  if (500 * rounds * d.lx1 + 6 * per_sm * warp_rows > 2100LL * d.lx1) return 0;  // ns
+  // four blocks per SM (a solving warp on each scheduler) where the columns fill them
+  const long long want = std::max<long long>(1, (std::min(per_sm, fit) + 3) / 4);
+  const long long most = std::max<long long>(1, (long long)((SM_BYTES / 4 - BLOCK_OVERHEAD) / luc_bytes(d.lx1)));
+  return (int)std::min<long long>(32, std::min(want, most));
+}
+
 int launch_diffusion_lu(const gem_grid* g, DiffArgs a, cudaStream_t st) {
   const Dims& d = g->dev.d;
   if (!a.lu) return set_err(GEM_EINVAL, "diffusion without a band-solve scratch");
   a.lu_slot = lu_slot_doubles(d.lx1);
   a.x3fast = (!g->dev.unit && g->dev.c3 == 0) ? 1 : 0;
+  const int cb = luc_columns(d);
+  if (cb > 0) {
+    const long long ng = ((long long)d.lx2 * d.lx3 + cb - 1) / cb;
+    const int warps = std::min(LUC_THREADS / 32, cb * ((d.lx1 + 31) / 32));
+    const size_t sm = luc_bytes(d.lx1) * cb;
+    auto kern = g->dev.unit ? k_diffusion_col<true> : k_diffusion_col<false>;
+    if (sm > 48 * 1024) GEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    kern<<<(unsigned)(ng * LSP), 32 * warps, sm, st>>>(a, cb);
+    GEM_LAUNCHED("k_diffusion_col");
+    return GEM_OK;
+  }
   const long long nblk = lu_slots_for(d) / LU_WPB;  // the work object holds this many slots
-  if (g->dev.unit)
-    k_diffusion_lu<true><<<(unsigned)nblk, 32 * LU_WPB, 0, st>>>(a);
-  else
-    k_diffusion_lu<false><<<(unsigned)nblk, 32 * LU_WPB, 0, st>>>(a);
+  const bool few = nblk <= (long long)num_sms() * LU_MINB_FEW;
+  auto kern = g->dev.unit ? (few ? k_diffusion_lu<true, LU_MINB_FEW> : k_diffusion_lu<true, LU_MINB>)
+                          : (few ? k_diffusion_lu<false, LU_MINB_FEW> : k_diffusion_lu<false, LU_MINB>);
+  kern<<<(unsigned)nblk, 32 * LU_WPB, 0, st>>>(a);
   GEM_LAUNCHED("k_diffusion_lu");
   return GEM_OK;
 }

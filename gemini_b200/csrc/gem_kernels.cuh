@@ -44,6 +44,8 @@ __constant__ double c_gammas[LSP] = {5.0 / 3, 7.0 / 5, 7.0 / 5, 7.0 / 5, 5.0 / 3
 #define GEM_G53 (5.0 / 3 - 1)
 #define GEM_G75 (7.0 / 5 - 1)
 __constant__ double c_gm1[LSP] = {GEM_G53, GEM_G75, GEM_G75, GEM_G75, GEM_G53, GEM_G53, GEM_G53};
+__constant__ double c_ygm1[LSP] = {1.0 / GEM_G53, 1.0 / GEM_G75, 1.0 / GEM_G75, 1.0 / GEM_G75,
+                                   1.0 / GEM_G53, 1.0 / GEM_G53, 1.0 / GEM_G53};
 __constant__ double c_gm1kb[LSP] = {GEM_G53 / KB, GEM_G75 / KB, GEM_G75 / KB, GEM_G75 / KB,
                                     GEM_G53 / KB, GEM_G53 / KB, GEM_G53 / KB};
 constexpr double QE = -1.0 * ELCHRG;
@@ -1408,7 +1410,7 @@ struct DiffArgs {
   int solver;  // 1 backward Euler, 2 TRBDF2
   int fused;   // 1: clean_param(3) + T2rhoe folded into the store
   double* lu;          // band-solve scratch of k_diffusion_lu (one slot per resident warp)
-  long long lu_slot;   // doubles per slot (>= lx1 * LU_ROW * 32)
+  long long lu_slot;   // doubles per slot (>= 32 lu_lane_doubles(lx1))
   int x3fast;          // column order of k_diffusion_lu: x3 fastest (x3-invariant metrics)
 };
 
@@ -1634,28 +1636,61 @@ __device__ __forceinline__ void band_solve_T(const WM& W, int M, int lane, RowM 
 //     (x1 column, species), a warp = 32 columns of one species.  Columns are enumerated x3
 //     fastest when the metric tables do not vary along x3 (the warp's metric loads are then
 //     one broadcast address), else x2 fastest.  Warp tasks run electrons first (their rows
-//     cost more).  Each resident warp owns a scratch slot of lx1 rows x LU_ROW doubles x 32
-//     lanes.
+//     cost more).  Each resident warp owns a scratch slot (LU_ROW_DEV doubles a row and the
+//     chunk checkpoints, times 32 lanes).
+//
+//     A thread walks along x1, the contiguous direction, so its own loads and stores of the
+//     state would touch 32 lines per warp access.  The warp moves T and n in, and T and
+//     rhoes out, through shared tiles of LU_TILE rows x 32 columns instead: 8 lanes per column
+//     copy 64 contiguous bytes, the next tile in flight (cp.async) while this one is used.
+//
+//     Bound by instruction issue and fixed latencies at 16 warps per SM (issue 40%, DRAM 35%
+//     of peak, 734 instructions per row and species of which 198 FP64).  At 384x192x192: 4.7
+//     ms; 7.1 ms with the factor rows kept in the scratch (28 doubles a row and species
+//     moved, not 21), each lane loading its own column, a branch per pivot choice and per
+//     exact quotient.
 // ======================================================================================
 constexpr int LU_WPB = 4;  // warps per block
-#ifndef GEM_LU_MINB
-#define GEM_LU_MINB 4  // resident blocks per SM the register budget is sized for
-#endif
-constexpr int LU_MINB_DEFAULT = GEM_LU_MINB;
+constexpr int LU_MINB = 4;        // resident blocks per SM the register budget is sized for
+// The same where the tasks do not fill more than this: no spills and more loads ahead of use
+// (128x64x64: 288 us against 320), while a grid that fills four needs them (64x96x96: 206
+// against 270).
+constexpr int LU_MINB_FEW = 3;
+constexpr int LU_ROW_DEV = 4;  // scratch doubles per row and lane: q-, q+, rhs, bq
 
-// column accessor of one thread (gemd::lu_column): four column offsets; the table base
-// addresses stay in the launch parameters (DiffArgs), so they cost no registers
+// rows of a scratch slot: the chunk copies may read up to LU_K rows past the last one
+__host__ __device__ __forceinline__ int lu_rows(int n) { return n + gemd::LU_K; }
+// scratch doubles of one lane for a column of n rows
+__host__ __device__ __forceinline__ long long lu_lane_doubles(int n) {
+  return (long long)lu_rows(n) * LU_ROW_DEV + 3LL * ((n + gemd::LU_K - 1) / gemd::LU_K);
+}
+
+// column accessor of one thread (gemd::lu_column): the state through the warp's tiles; the
+// table base addresses stay in the launch parameters (DiffArgs), so they cost no registers
+constexpr int LU_TW = gemd::LU_TILE + 1;  // tile row pitch: lanes on distinct bank pairs
+constexpr int LU_TN = 32 * LU_TW;         // doubles of a tile
+struct alignas(16) LuTiles {
+  // T and n of tile buffer b at t[b]; after the first forward pass buffer 1 holds the next
+  // chunk's scratch lines and buffer 0 the rows being stored
+  double t[2][2 * LU_TN];
+  long long ofs[32];   // ghosted offset of cell 0 of each column
+  long long iofs[32];  // interior offset of cell 1, minus 1
+};
+
 template <bool UNIT>
 struct LuAccDev {
   const DiffArgs& P;
-  long long tofs;  // Ts(s) + tofs: cell 0 of the column (ghosted block); ns(s) at nofs
-  long long nofs;
+  const double *tT, *tn;  // this lane's row of tile 0 of T and n
   long long mofs;  // cell 0 in the metric tables
   long long qofs;  // interior offset of cell 1, minus 1 (neutral densities)
   long long jofs;  // cell 0 in J1 (ghosted)
-  double* sc;      // this lane's scratch: row i, slot k at sc[((i-1)*LU_ROW + k)*32]
-  __device__ __forceinline__ double T(int i) const { return P.B.F[tofs + i]; }
-  __device__ __forceinline__ double n(int i) const { return __ldg(P.B.F + nofs + i); }
+  double* sc;      // this lane's scratch: row i, slot k at sc[((i-1)*LU_ROW_DEV + k)*32]
+  double* cp;      // this lane's checkpoints: chunk c, value k at cp[(c*3 + k)*32]
+  __device__ __forceinline__ static int tslot(int i) {
+    return (((i - 1) / gemd::LU_TILE) & 1) * (2 * LU_TN) + ((i - 1) & (gemd::LU_TILE - 1));
+  }
+  __device__ __forceinline__ double T(int i) const { return tT[tslot(i)]; }
+  __device__ __forceinline__ double n(int i) const { return tn[tslot(i)]; }
   __device__ __forceinline__ void metrics(int i, double& a1, double& a2, double& a3, double& y1, double& ha,
                                           double& yha) const {
     const long long k = mofs + i;
@@ -1679,53 +1714,130 @@ struct LuAccDev {
   __device__ __forceinline__ double ydxi(int i) const { return __ldg(P.G.L[0].ydxi + i - 1); }
   __device__ __forceinline__ double dxs(int i) const { return __ldg(P.G.L[0].dxs + i); }
   __device__ __forceinline__ double ydxs(int i) const { return __ldg(P.G.L[0].ydxs + i); }
-  // the scratch streams through L2 only (ld/st.global.cg), keeping L1 for the column inputs
-  // and the grid tables the warp re-reads
-  __device__ __forceinline__ double sld(int i, int k) const { return __ldcg(sc + ((i - 1) * gemd::LU_ROW + k) * 32); }
-  __device__ __forceinline__ void sst(int i, int k, double v) const {
-    __stcg(sc + ((i - 1) * gemd::LU_ROW + k) * 32, v);
+  // the scratch streams through L2 only (ld/st.global.cg), keeping L1 for the grid tables the
+  // warp re-reads
+  __device__ __forceinline__ double* at(int i, int k) const {
+    if (k < gemd::LU_CP) return sc + ((i - 1) * LU_ROW_DEV + k) * 32;
+    return cp + ((i - 1) / gemd::LU_K * 3 + (k - gemd::LU_CP)) * 32;
+  }
+  __device__ __forceinline__ double sld(int i, int k) const { return __ldcg(at(i, k)); }
+  __device__ __forceinline__ void sst(int i, int k, double v) const { __stcg(at(i, k), v); }
+};
+
+// asynchronous 16-byte copy through L2 only
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+
+// The warp's copies: tiles of the state (8 lanes per column, 4 columns per pass) and chunks of
+// the scratch (16 lanes per 256-byte line, 2 lines per pass).
+struct LuTileIo {
+  LuTiles& W;
+  const double *T, *n;  // species blocks
+  const double* slot;   // the warp's scratch
+  int lx1;
+  __device__ __forceinline__ void issue(const double* src, double* dst, int i0) const {
+    const int lane = threadIdx.x & 31;
+    const int r = lane & (gemd::LU_TILE - 1), c0 = lane / gemd::LU_TILE;
+    if (i0 + r <= lx1) {
+#pragma unroll
+      for (int c = c0; c < 32; c += 32 / gemd::LU_TILE) cp_async8(dst + c * LU_TW + r, src + W.ofs[c] + i0 + r);
+    }
+  }
+  __device__ __forceinline__ void issue_in(int i0) const {
+    const int b = ((i0 - 1) / gemd::LU_TILE) & 1;
+    if (i0 <= lx1) {
+      issue(T, W.t[b], i0);
+      issue(n, W.t[b] + LU_TN, i0);
+    }
+    cp_async_commit();
+  }
+  // cells i0 .. i0+LU_TILE-1 readable; the other buffer, last read before this call, refills
+  __device__ __forceinline__ void tile(int i0) const {
+    cp_async_wait<0>();
+    __syncwarp();
+    issue_in(i0 + gemd::LU_TILE);
+  }
+  // chunk lines in buffer 1: line k*LU_K + q = slot k of row q of the chunk
+  template <bool ELEC>
+  __device__ __forceinline__ void request(int iq, int iv) const {
+    static_assert((ELEC ? 4 : 3) * gemd::LU_K * 32 <= 2 * LU_TN && gemd::LU_K % 2 == 0, "chunk buffer");
+    const int lane = threadIdx.x & 31;
+    const double* src = slot + ((iq - 1 + (lane >> 4)) * LU_ROW_DEV) * 32 + (lane & 15) * 2;
+    const double* srv = slot + ((iv - 1 + (lane >> 4)) * LU_ROW_DEV) * 32 + (lane & 15) * 2;
+    double* dst = W.t[1] + lane * 2;
+    __syncwarp();  // the buffer's last readers are done, and the scratch is written
+#pragma unroll
+    for (int k = 0; k < (ELEC ? 4 : 3); ++k)
+#pragma unroll
+      for (int q = 0; q < gemd::LU_K; q += 2)
+        cp_async16(dst + (k * gemd::LU_K + q) * 32, (k == gemd::LU_RHS ? srv : src) + (q * LU_ROW_DEV + k) * 32);
+    cp_async_commit();
+  }
+  template <bool ELEC, class Acc>
+  __device__ __forceinline__ gemd::LuRows take(const Acc&, int) const {
+    const double* b = W.t[1] + (threadIdx.x & 31);
+    cp_async_wait<0>();
+    __syncwarp();
+    gemd::LuRows w;
+#pragma unroll
+    for (int q = 0; q < gemd::LU_K; ++q) {
+      w.qm[q] = b[(gemd::LU_QM * gemd::LU_K + q) * 32];
+      w.qp[q] = b[(gemd::LU_QP * gemd::LU_K + q) * 32];
+      w.v[q] = b[(gemd::LU_RHS * gemd::LU_K + q) * 32];
+      w.bq[q] = ELEC ? b[(gemd::LU_BQ * gemd::LU_K + q) * 32] : 0.0;
+    }
+    return w;
   }
 };
 
 // The solution's destination: max(T,100) (multifluid.f90:340) into Ts; fused with
-// clean_param(3) (null cells 100) and T2rhoe (rhoes from ns), whose inputs are loaded ahead.
-struct LuPre {
-  double nv;
-  bool nul;
-};
+// clean_param(3) (null cells 100) and T2rhoe (rhoes from ns).  The rows arrive from the last to
+// the first: each lane collects its column in the T part of buffer 0 and the warp stores a
+// tile when its first row is in, with n of the same rows, requested with its last row.
 struct LuStoreDev {
-  double* Tout;
-  double* re;                 // rhoes of the column (fused), else null
-  const double* nc;           // ns of the column
-  const unsigned char* nul;   // null-point flags of the column (interior offset - 1), or null
-  int s;
-  __device__ __forceinline__ LuPre pre(int i) const {
-    LuPre p;
-    p.nv = re ? __ldg(nc + i) : 0.0;
-    p.nul = nul ? nul[i] != 0 : false;
-    return p;
+  const LuTileIo& io;
+  double* Tout;               // species block
+  double* re;                 // rhoes block (fused), else null
+  const unsigned char* nul;   // null-point flags, or null
+  int s, ncols;               // columns of this warp that exist
+  __device__ __forceinline__ int pre(int) const { return 0; }
+  __device__ __forceinline__ void operator()(int i, double x, int) const {
+    const int r = (i - 1) & (gemd::LU_TILE - 1);
+    if (re && (r == gemd::LU_TILE - 1 || i == io.lx1)) {
+      io.issue(io.n, io.W.t[0] + LU_TN, i - r);
+      cp_async_commit();
+    }
+    io.W.t[0][(threadIdx.x & 31) * LU_TW + r] = x;
+    if (r == 0) flush(i);
   }
-  __device__ __forceinline__ void operator()(int i, double x, const LuPre& p) const {
-    double T = fmax_f(x, 100.0);
-    if (p.nul) T = 100;
-    Tout[i] = T;
-    if (re) re[i] = p.nv * KB * T / (c_gammas[s] - 1);  // T2rhoe (multifluid.f90:193-202)
+  __device__ __forceinline__ void flush(int i0) const {
+    const int lane = threadIdx.x & 31;
+    const int r = lane & (gemd::LU_TILE - 1), c0 = lane / gemd::LU_TILE;
+    if (re) cp_async_wait<0>();
+    __syncwarp();
+    const int i = i0 + r;
+    if (i <= io.lx1) {
+#pragma unroll
+      for (int c = c0; c < 32; c += 32 / gemd::LU_TILE) {
+        if (c < ncols) {
+          double T = fmax_f(io.W.t[0][c * LU_TW + r], 100.0);
+          if (nul && nul[io.W.iofs[c] + i]) T = 100;
+          const long long k = io.W.ofs[c] + i;
+          Tout[k] = T;
+          // T2rhoe (multifluid.f90:193-202): n*kB*T/(gamma-1)
+          if (re) re[k] = mdiv(io.W.t[0][LU_TN + c * LU_TW + r] * KB * T, c_gm1[s], c_ygm1[s]);
+        }
+      }
+    }
+    __syncwarp();
   }
 };
 
-// One warp task: 32 columns of one species.  slot = this warp's scratch slot (lane 0).
-template <bool UNIT>
-__device__ __forceinline__ void b_diffusion_lu(const DiffArgs& P, int task, double* slot) {
-  const GridDev& G = P.G;
-  const Dims d = G.d;
-  const int n = d.lx1;
-  const int lane = threadIdx.x & 31;
-  const int ncol = d.lx2 * d.lx3;
-  const int tps = (ncol + 31) / 32;
-  const int s = LSP - 1 - task / tps;
-  const int col = (task % tps) * 32 + lane;
-  if (col >= ncol) return;
-  int i2, i3;
+// Column (i2, i3) of index col in the launch's column order.
+__device__ __forceinline__ void lu_column_at(const DiffArgs& P, int col, int& i2, int& i3) {
+  const Dims& d = P.G.d;
   if (P.x3fast) {
     i3 = col % d.lx3 + 1;
     i2 = col / d.lx3 + 1;
@@ -1733,59 +1845,295 @@ __device__ __forceinline__ void b_diffusion_lu(const DiffArgs& P, int task, doub
     i2 = col % d.lx2 + 1;
     i3 = col / d.lx2 + 1;
   }
-  const long long m0 = gi(d, 0, i2, i3);
-  const long long mm0 = cmi(G, 0, i2, i3);
-  const long long q0 = ci(d, 1, i2, i3) - 1;
+}
 
-  LuAccDev<UNIT> a{P, (long long)(4 * LSP + s) * d.ng + m0, (long long)s * d.ng + m0, mm0, q0, m0, slot + lane};
-  // Dirichlet values (diffusion.f90:54-79): the exospheric side takes Teinf or the column's value
-  const double tn1 = __ldg(P.Tn + ci(d, 1, i2, i3)), tnl = __ldg(P.Tn + ci(d, n, i2, i3));
+// Constants of one (column, species); the Dirichlet values (diffusion.f90:54-79): the
+// exospheric side takes Teinf or the column's value.
+__device__ __forceinline__ gemd::LuK lu_consts(const DiffArgs& P, int s, int i2, int i3) {
+  const Dims& d = P.G.d;
+  const double tn1 = __ldg(P.Tn + ci(d, 1, i2, i3)), tnl = __ldg(P.Tn + ci(d, d.lx1, i2, i3));
   const double tinf = P.Ttop ? __ldg(P.Ttop + (i2 - 1) + (long long)d.lx2 * (i3 - 1)) : P.Teinf;
   gemd::LuK k;
-  k.n = n;
+  k.n = d.lx1;
   k.s = s;
   k.dt = *P.dtp;
-  if (G.gridflag == 0) {
-    k.tmin = tn1;
-    k.tmax = tnl;
-  } else if (G.gridflag == 1) {
-    k.tmin = tinf;
-    k.tmax = tnl;
-  } else {
-    k.tmin = tn1;
-    k.tmax = tinf;
-  }
+  k.tmin = P.G.gridflag == 1 ? tinf : tn1;
+  k.tmax = (P.G.gridflag == 0 || P.G.gridflag == 1) ? tnl : tinf;
   k.c0 = (c_gammas[s] - 1.0) / KB;
   k.tcoef = (s < LSP - 1) ? c_tcoef[s] : 0.0;
-  LuStoreDev st;
-  st.Tout = P.B.Ts(s) + m0;
-  st.re = P.fused ? P.B.re(s) + m0 : nullptr;
-  st.nc = P.B.ns(s) + m0;
-  st.nul = (P.fused && G.has_null) ? G.nullpts + (ci(d, 1, i2, i3) - 1) : nullptr;
-  st.s = s;
+  return k;
+}
+
+// One warp task: 32 columns of one species.  slot = this warp's scratch slot (lane 0).
+template <bool UNIT>
+__device__ __forceinline__ void b_diffusion_lu(const DiffArgs& P, int task, double* slot, LuTiles& W) {
+  const GridDev& G = P.G;
+  const Dims d = G.d;
+  const int n = d.lx1;
+  const int lane = threadIdx.x & 31;
+  const int ncol = d.lx2 * d.lx3;
+  const int tps = (ncol + 31) / 32;
+  const int s = LSP - 1 - task / tps;
+  const int col0 = (task % tps) * 32;
+  // lanes past the last column repeat it (their stores are left out)
+  const int col = (col0 + lane < ncol) ? col0 + lane : ncol - 1;
+  int i2, i3;
+  lu_column_at(P, col, i2, i3);
+  const long long m0 = gi(d, 0, i2, i3);
+  const long long q0 = ci(d, 1, i2, i3) - 1;
+  W.ofs[lane] = m0;
+  W.iofs[lane] = q0;
+  __syncwarp();
+  const LuTileIo io{W, P.B.Ts(s), P.B.ns(s), slot, n};
+  io.issue_in(1);
+
+  const LuAccDev<UNIT> a{P, W.t[0] + lane * LU_TW, W.t[0] + LU_TN + lane * LU_TW, cmi(G, 0, i2, i3), q0, m0, slot + lane,
+                         slot + (long long)lu_rows(n) * LU_ROW_DEV * 32 + lane};
+  const gemd::LuK k = lu_consts(P, s, i2, i3);
+  const LuStoreDev st{io, P.B.Ts(s), P.fused ? P.B.re(s) : nullptr, (P.fused && G.has_null) ? G.nullpts : nullptr, s,
+                      ncol - col0};
   if (s == LSP - 1)
-    gemd::lu_column<UNIT, true>(a, k, P.solver, st);
+    gemd::lu_column<UNIT, true>(a, k, P.solver, st, io);
   else
-    gemd::lu_column<UNIT, false>(a, k, P.solver, st);
-  double* Tout = st.Tout;
-  if (!P.fused) {
+    gemd::lu_column<UNIT, false>(a, k, P.solver, st, io);
+  if (!P.fused && col0 + lane < ncol) {
+    double* Tout = st.Tout + m0;
     Tout[0] = fmax_f(k.tmin, 100.0);
     Tout[n + 1] = fmax_f(k.tmax, 100.0);
   }
+  __syncwarp();  // the tiles and offsets are free for the warp's next task
 }
 
 // plain launch: persistent warps over the warp tasks; scratch slot = the global warp index
-template <bool UNIT>
-__global__ void __launch_bounds__(32 * LU_WPB, GEM_LU_MINB) k_diffusion_lu(DiffArgs P) {
+template <bool UNIT, int MINB>
+__global__ void __launch_bounds__(32 * LU_WPB, MINB) k_diffusion_lu(DiffArgs P) {
+  __shared__ LuTiles tiles[LU_WPB];
   const int warp = threadIdx.x >> 5;
   const int gw = blockIdx.x * LU_WPB + warp;
   const int nw = gridDim.x * LU_WPB;
   const int ncol = P.G.d.lx2 * P.G.d.lx3;
   const int ntask = ((ncol + 31) / 32) * LSP;
   double* slot = P.lu + (long long)gw * P.lu_slot;
-  for (int t = gw; t < ntask; t += nw) b_diffusion_lu<UNIT>(P, t, slot);
+  for (int t = gw; t < ntask; t += nw) b_diffusion_lu<UNIT>(P, t, slot, tiles[warp]);
 }
 
+
+// The same solve for grids with few columns, whose time is one thread's serial chain: a block
+// holds cb columns of one species in shared memory, all threads form the band rows
+// (lanes along x1, coalesced) and only the elimination and the back substitution run one
+// thread per column, in place over five row arrays.  The factors q-, q+, bq wait in the
+// scratch (in L2 at these sizes) for the BDF2 rows.  Bound by the solving threads' chain (two
+// passes of about 200 and 100 cycles a row and stage).  64x8x6: 33 us, 120 by k_diffusion_lu;
+// 96x32x32: 76, 182; 192x96x1 backward Euler: 46, 290.
+//   doubles per row: 0 C / s / u0, 1 B / d / u1, 2 e / u2, 3 r / y / x, 4 D / 1/u0
+// Five consecutive doubles a row (an odd number) and an odd column pitch keep both kinds of
+// access on distinct bank pairs, and one pointer with fixed offsets serves a row.
+constexpr int LUC_ROW = 5;
+constexpr int LUC_THREADS = 128;
+__host__ __device__ __forceinline__ int luc_pitch(int n) { return (LUC_ROW * n) | 1; }
+
+// Elimination and back substitution of one column's band rows, in place (rows 2..n given).
+__device__ __forceinline__ void luc_solve(const gemd::LuK& k, double* W) {
+  const int n = k.n;
+  gemd::LuState st{1.0, 0.0, k.tmin};
+  gemd::BandRow w{W[5], W[6], W[7], W[8]};
+  double* p = W;  // row j
+#pragma unroll 1
+  for (int j = 1; j < n; ++j, p += LUC_ROW) {
+    const gemd::BandRow cur = w;
+    if (j + 1 < n) w = gemd::BandRow{p[10], p[11], p[12], p[13]};
+    const gemd::LuU u = gemd::lu_step(st, cur);
+    p[0] = u.u0;
+    p[1] = u.u1;
+    p[2] = u.u2;
+    p[3] = u.y;
+    p[4] = u.rec;
+  }
+  double x1 = gemd::qdiv(st.b, st.p, gemd::rcp_rn(st.p)), x2 = 0.0;
+  p[3] = x1;
+  p -= LUC_ROW;  // row n-1
+  double u0 = p[0], u1 = p[1], u2 = 0.0, y = p[3], rec = p[4];
+#pragma unroll 1
+  for (int i = n - 1; i >= 1; --i, p -= LUC_ROW) {
+    double v0 = 0.0, v1 = 0.0, v2 = 0.0, vy = 0.0, vr = 0.0;
+    if (i > 1) {
+      v0 = p[-5];
+      v1 = p[-4];
+      v2 = p[-3];
+      vy = p[-2];
+      vr = p[-1];
+    }
+    double x = y;
+    if (i <= n - 2) x = x - x2 * u2;
+    x = x - x1 * u1;
+    x = gemd::qdiv(x, u0, rec);
+    p[3] = x;
+    x2 = x1;
+    x1 = x;
+    u0 = v0;
+    u1 = v1;
+    u2 = v2;
+    y = vy;
+    rec = vr;
+  }
+}
+
+// cell and row accessors of the row-parallel phases
+template <bool UNIT>
+struct LucAcc {
+  const DiffArgs& P;
+  long long mofs, qofs, jofs;
+  __device__ __forceinline__ void metrics(int i, double& a1, double& a2, double& a3, double& y1, double& ha,
+                                          double& yha) const {
+    const long long k = mofs + i;
+    a1 = __ldg(P.G.h1 + k);
+    a2 = __ldg(P.G.h2 + k);
+    a3 = __ldg(P.G.h3 + k);
+    y1 = __ldg(P.G.yh1 + k);
+    ha = __ldg(P.G.ha1_0 + k);
+    yha = __ldg(P.G.yha1_0 + k);
+  }
+  __device__ __forceinline__ double dx(int i) const { return __ldg(P.G.L[0].dx + i); }
+  __device__ __forceinline__ double ydx(int i) const { return __ldg(P.G.L[0].ydx + i); }
+  __device__ __forceinline__ double dxi(int i) const { return __ldg(P.G.L[0].dxi + i - 1); }
+  __device__ __forceinline__ double ydxi(int i) const { return __ldg(P.G.L[0].ydxi + i - 1); }
+  __device__ __forceinline__ double dxs(int i) const { return __ldg(P.G.L[0].dxs + i); }
+  __device__ __forceinline__ double ydxs(int i) const { return __ldg(P.G.L[0].ydxs + i); }
+};
+
+template <bool UNIT, bool ELEC, int STG1>
+__device__ __forceinline__ void b_diffusion_col(const DiffArgs& P, int s, int col0, int cb, double* W, double* sc) {
+  const Dims& d = P.G.d;
+  const int n = d.lx1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int pitch = luc_pitch(n), nch = (n + 31) / 32;
+  const double* T = P.B.Ts(s);
+  const double* nv = P.B.ns(s);
+  const long long nc = nci(d);
+  const double dt = *P.dtp;
+  // warp items: (column, 32 rows)
+  auto each = [&](auto&& f) {
+    for (int it = warp; it < cb * nch; it += nwarp) {
+      const int c = it / nch;
+      const int i = (it - c * nch) * 32 + lane + 1;
+      int i2, i3;
+      lu_column_at(P, col0 + c, i2, i3);
+      if (i <= n) f(c, i, i2, i3, W + c * pitch + (i - 1) * LUC_ROW);
+    }
+    __syncthreads();
+  };
+  each([&](int, int i, int i2, int i3, double* w) {  // C, B, D of every cell
+    const long long m = gi(d, i, i2, i3);
+    const LucAcc<UNIT> a{P, cmi(P.G, 0, i2, i3), 0, 0};
+    gemd::CellIn cin;
+    cin.T = T[m];
+    cin.n = __ldg(nv + m);
+    cin.n1 = cin.n2 = cin.n3 = cin.j1 = 0.0;
+    if (ELEC) {
+      const long long q = ci(d, i, i2, i3);
+      cin.n1 = __ldg(P.nn + q);
+      cin.n2 = __ldg(P.nn + nc + q);
+      cin.n3 = __ldg(P.nn + 2 * nc + q);
+      cin.j1 = __ldg(P.J1 + m);
+    }
+    gemd::LuK k;
+    k.c0 = (c_gammas[s] - 1.0) / KB;
+    k.tcoef = ELEC ? 0.0 : c_tcoef[s];
+    const gemd::Coef f = gemd::cell_coef<UNIT, ELEC>(a, k, i, cin);
+    w[0] = f.C;
+    w[1] = f.B;
+    w[4] = f.D;
+  });
+  const gemd::StageDt<STG1> t(dt);
+  each([&](int c, int i, int i2, int i3, double* w) {  // factors and the first stage's rows
+    gemd::BandRow r{0.0, 1.0, 0.0, 0.0};
+    if (i == 1) return;
+    if (i < n) {
+      const LucAcc<UNIT> a{P, 0, 0, 0};
+      const gemd::RowFac f = gemd::row_factors<ELEC>(a, i, w[0], w[1], w[4 - LUC_ROW], w[4], w[4 + LUC_ROW]);
+      const double* Tc = T + gi(d, i, i2, i3);
+      r = gemd::band_row<STG1>(t, f.qm, f.qp, f.bq, Tc[-1], Tc[0], Tc[1],
+                               STG1 == gemd::ST_BE ? gemd::qdiv(Tc[0], t.h, t.y) : 0.0);
+      if (STG1 == gemd::ST_TR) {
+        double* q = sc + (long long)c * 3 * n + (i - 1);
+        __stcg(q, f.qm);
+        __stcg(q + n, f.qp);
+        if (ELEC) __stcg(q + 2 * n, f.bq);
+      }
+    } else {
+      r.r = lu_consts(P, s, i2, i3).tmax;
+    }
+    w[0] = r.s;
+    w[1] = r.d;
+    w[2] = r.e;
+    w[3] = r.r;
+  });
+  // the column threads: the warp differs from block to block, so that co-resident blocks use
+  // different schedulers
+  const int cw = blockIdx.x % nwarp;
+  auto solve = [&]() {
+    if (warp == cw && lane < cb) {
+      int i2, i3;
+      lu_column_at(P, col0 + lane, i2, i3);
+      luc_solve(lu_consts(P, s, i2, i3), W + lane * pitch);
+    }
+    __syncthreads();
+  };
+  solve();
+  if (STG1 == gemd::ST_TR) {
+    const gemd::StageDt<gemd::ST_BDF2> t3(dt);
+    each([&](int c, int i, int i2, int i3, double* w) {
+      if (i == 1) return;
+      gemd::BandRow r{0.0, 1.0, 0.0, 0.0};
+      if (i < n) {
+        const double* q = sc + (long long)c * 3 * n + (i - 1);
+        const double rhs = gemd::bdf2_rhs(t3, T[gi(d, i, i2, i3)], w[3]);
+        r = gemd::band_row<gemd::ST_BDF2>(t3, __ldcg(q), __ldcg(q + n), ELEC ? __ldcg(q + 2 * n) : 0.0, 0.0, 0.0, 0.0,
+                                          rhs);
+      } else {
+        r.r = lu_consts(P, s, i2, i3).tmax;
+      }
+      w[0] = r.s;
+      w[1] = r.d;
+      w[2] = r.e;
+      w[3] = r.r;
+    });
+    solve();
+  }
+  // max(T,100); fused: clean_param(3)'s null cells and T2rhoe, as LuStoreDev
+  double* Tout = P.B.Ts(s);
+  double* re = P.fused ? P.B.re(s) : nullptr;
+  each([&](int, int i, int i2, int i3, double* w) {
+    const long long m = gi(d, i, i2, i3);
+    double Tn = fmax_f(w[3], 100.0);
+    if (re && is_null(P.G, i, i2, i3)) Tn = 100;
+    Tout[m] = Tn;
+    if (re) re[m] = mdiv(__ldg(nv + m) * KB * Tn, c_gm1[s], c_ygm1[s]);
+    if (!re && (i == 1 || i == n)) {
+      const gemd::LuK k = lu_consts(P, s, i2, i3);
+      if (i == 1) Tout[m - 1] = fmax_f(k.tmin, 100.0);
+      if (i == n) Tout[m + 1] = fmax_f(k.tmax, 100.0);
+    }
+  });
+}
+
+template <bool UNIT>
+__global__ void __launch_bounds__(LUC_THREADS, 4) k_diffusion_col(DiffArgs P, int cb) {
+  extern __shared__ double luc_w[];
+  const int ncol = P.G.d.lx2 * P.G.d.lx3;
+  const int ng = (ncol + cb - 1) / cb;
+  const int s = LSP - 1 - blockIdx.x / ng;
+  const int col0 = (blockIdx.x % ng) * cb;
+  const int nb = ncol - col0 < cb ? ncol - col0 : cb;
+  double* sc = P.lu + ((long long)s * ncol + col0) * 3 * P.G.d.lx1;  // 3 lx1 doubles per column
+  if (s == LSP - 1) {
+    if (P.solver == 2) b_diffusion_col<UNIT, true, gemd::ST_TR>(P, s, col0, nb, luc_w, sc);
+    else b_diffusion_col<UNIT, true, gemd::ST_BE>(P, s, col0, nb, luc_w, sc);
+  } else {
+    if (P.solver == 2) b_diffusion_col<UNIT, false, gemd::ST_TR>(P, s, col0, nb, luc_w, sc);
+    else b_diffusion_col<UNIT, false, gemd::ST_BE>(P, s, col0, nb, luc_w, sc);
+  }
+}
 
 // standalone energy_diffusion: max(T,100) on the ghost cells other than the x1 BC layers
 __global__ void k_diffusion_ghost_floor(GridDev G, Blocks B) {
