@@ -83,12 +83,12 @@ __global__ void __launch_bounds__(128) kb_ghost_x3(const InstDev* __restrict__ i
   }
 }
 
-template <int DIM, bool UNIT>
+template <int DIM, bool UNIT, bool INV = false>
 __global__ void __launch_bounds__(224, 2) kb_sweep_march(const InstDev* __restrict__ inst, const Item* __restrict__ it, int n) {
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     const Item q = it[w];
     const InstDev& I = inst[q.x];
-    b_sweep_march<DIM, UNIT, true>(I.sw, VB{q.y, q.z, q.w});
+    b_sweep_march<DIM, UNIT, true, 2, false, INV>(I.sw, VB{q.y, q.z, q.w});
     if (DIM == 2) __syncthreads();  // the epilogue's shared buffers are reused by the next item
   }
 }
@@ -152,6 +152,7 @@ enum BatchKernel { BK_DT = 0, BK_GX1, BK_GX2, BK_GX3, BK_SW3, BK_SW1, BK_SW2, BK
 struct BatchLaunch {
   int kernel = 0;
   int unit = 0;
+  bool inv = true;  // every instance's metrics are x3-invariant (x3 sweep)
   int grid = 0;
   std::vector<Item> items;
   Item* d_items = nullptr;
@@ -211,6 +212,7 @@ int launch_grid(gem_batch* b, BatchLaunch& L) {
     case BK_GX2: return occupancy_grid(kb_ghost_x2, 128, 0, n, sc, &L.grid);
     case BK_GX3: return occupancy_grid(kb_ghost_x3, 128, 0, n, sc, &L.grid);
     case BK_SW3: return u ? occupancy_grid(kb_sweep_march<3, true>, 32 * LSP, 0, n, sc, &L.grid)
+             : L.inv      ? occupancy_grid(kb_sweep_march<3, false, true>, 32 * LSP, 0, n, sc, &L.grid)
                           : occupancy_grid(kb_sweep_march<3, false>, 32 * LSP, 0, n, sc, &L.grid);
     case BK_SW1: return u ? occupancy_grid(kb_sweep_x1<true>, 32 * LSP, 0, n, sc, &L.grid)
                           : occupancy_grid(kb_sweep_x1<false>, 32 * LSP, 0, n, sc, &L.grid);
@@ -260,10 +262,15 @@ int batch_build_lists(gem_batch* b) {
           case BK_DT:
             add_items(launch_for(k, u), i, std::min<long long>((long long)d.lx2 * d.lx3, (long long)num_sms() * 8));
             break;
-          case BK_GX1: add_items(launch_for(k, 0), i, grid_for((long long)(d.lx2 + 4) * (d.lx3 + 4) * LSP, 128)); break;
+          case BK_GX1: add_items(launch_for(k, 0), i, grid_for(ghost_x1_items(d, g->dev.flagper, LSP, true), 128)); break;
           case BK_GX2: add_items(launch_for(k, 0), i, grid_for((long long)(d.lx1 + 4) * (d.lx3 + 4) * LSP, 128)); break;
           case BK_GX3: add_items(launch_for(k, 0), i, grid_for((long long)(d.lx1 + 4) * (d.lx2 + 4) * LSP, 128)); break;
-          case BK_SW3: add_items(launch_for(k, u), i, gx13, d.lx2); break;
+          case BK_SW3: {
+            BatchLaunch& L = launch_for(k, u);
+            L.inv = L.inv && g->dev.c3 == 0;
+            add_items(L, i, gx13, d.lx2);
+            break;
+          }
           case BK_SW1: add_items(launch_for(k, u), i, d.lx2, d.lx3); break;
           case BK_SW2: add_items(launch_for(k, u), i, gx13, d.lx3); break;
           case BK_EPI: add_items(launch_for(k, 0), i, grid_for(ghost_cells(d), 256)); break;
@@ -327,6 +334,7 @@ int batch_enqueue(gem_batch* b, cudaStream_t st, bool fixed_dt = false) {
       case BK_GX3: kb_ghost_x3<<<L.grid, 128, 0, st>>>(I, L.d_items, n); break;
       case BK_SW3:
         if (u) kb_sweep_march<3, true><<<L.grid, dim3(32, LSP), 0, st>>>(I, L.d_items, n);
+        else if (L.inv) kb_sweep_march<3, false, true><<<L.grid, dim3(32, LSP), 0, st>>>(I, L.d_items, n);
         else kb_sweep_march<3, false><<<L.grid, dim3(32, LSP), 0, st>>>(I, L.d_items, n);
         break;
       case BK_SW1:

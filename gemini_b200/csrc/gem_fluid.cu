@@ -109,6 +109,7 @@ struct gem_work {
   double *vs1i, *vs2i, *vs3i, *nn, *Tn, *dt;
   double* Ttop;             // per-column exospheric temperature (lx2*lx3), or null for Teinf
   double* lu;               // band-solve scratch of k_diffusion_lu (lu_slots() slots of lx1 rows)
+  double* sweep;            // out-of-place blocks of the fused sweeps on small grids
   // the reference work object's sub-step contents for the host-memory *_C routines, allocated
   // on first use: the neutral state and ionization rates (gem_work_set_sources) and the
   // artificial viscosity Q, production and loss rates Pr, Lo
@@ -159,6 +160,33 @@ int check_step(const gem_grid* g) {
   return GEM_OK;
 }
 
+// Parts of a line in the fused x2 / x3 sweeps.  A thread marches along its line, about 1.3 us a
+// cell however few lines there are, so lines are cut until two blocks per SM have work, but
+// not below four cells (a part repeats two positions).  1 for both: the sweeps run in place.
+int sweep_parts(const Dims& d, int dim) {
+  const int lx = dim == 3 ? d.lx3 : d.lx2, other = dim == 3 ? d.lx2 : d.lx3;
+  const long long blocks = (long long)((d.lx1 + 31) / 32) * other;
+  return (int)std::max<long long>(1, std::min<long long>(2LL * num_sms() / blocks, lx / 4));
+}
+
+// The out-of-place blocks of the fused sweeps where a line is cut (else null): densities,
+// momentum and energy densities of all species, allocated by the first step.
+int work_sweeps(gem_work* w, const gem_grid* g, SweepArgs& a) {
+  const Dims& d = g->dev.d;
+  if (sweep_parts(d, 2) == 1 && sweep_parts(d, 3) == 1) return GEM_OK;
+  if (!w->sweep) {
+    const size_t bytes = sizeof(double) * 3 * LSP * d.ng;
+    if (cudaMalloc(&w->sweep, bytes) != cudaSuccess) {
+      w->sweep = nullptr;
+      return set_err(GEM_ENOMEM, "cudaMalloc of %zu bytes for the sweeps' scratch failed", bytes);
+    }
+  }
+  a.nsB = w->sweep;
+  a.rvB = a.nsB + LSP * d.ng;
+  a.reB = a.rvB + LSP * d.ng;
+  return GEM_OK;
+}
+
 template <int DIM, bool FUSED>
 int launch_sweep_t(const gem_grid* g, SweepArgs a, int nsp, cudaStream_t st) {
   const Dims& d = g->dev.d;
@@ -166,22 +194,29 @@ int launch_sweep_t(const gem_grid* g, SweepArgs a, int nsp, cudaStream_t st) {
   if (DIM == 1) {
     // one warp per (x1 column, species)
     dim3 grid(d.lx2, d.lx3);
-    if (g->dev.unit)
+    if (FUSED && a.nsB) {
+      if (g->dev.unit) k_sweep_x1<true, FUSED, FUSED><<<grid, block, 0, st>>>(a);
+      else k_sweep_x1<false, FUSED, FUSED><<<grid, block, 0, st>>>(a);
+    } else if (g->dev.unit) {
       k_sweep_x1<true, FUSED><<<grid, block, 0, st>>>(a);
-    else
+    } else {
       k_sweep_x1<false, FUSED><<<grid, block, 0, st>>>(a);
+    }
     GEM_LAUNCHED("k_sweep_x1");
     return GEM_OK;
   }
   // one thread per (x2 or x3 line, species), 32 adjacent x1 per warp
-  dim3 grid((d.lx1 + 31) / 32, (DIM == 3) ? d.lx2 : d.lx3);
+  dim3 grid((d.lx1 + 31) / 32, (DIM == 3) ? d.lx2 : d.lx3, FUSED && a.nsB ? sweep_parts(d, DIM) : 1);
   if (DIM == 3 && FUSED) {  // periodicity as a template parameter
     const bool per = g->dev.flagper != 0;
     if (g->dev.unit) {
       if (per) k_sweep_march<3, true, true, 1><<<grid, block, 0, st>>>(a);
       else k_sweep_march<3, true, true, 0><<<grid, block, 0, st>>>(a);
     } else {
-      if (per) k_sweep_march<3, false, true, 1><<<grid, block, 0, st>>>(a);
+      const bool inv = g->dev.c3 == 0;
+      if (per && inv) k_sweep_march<3, false, true, 1, false, true><<<grid, block, 0, st>>>(a);
+      else if (per) k_sweep_march<3, false, true, 1><<<grid, block, 0, st>>>(a);
+      else if (inv) k_sweep_march<3, false, true, 0, false, true><<<grid, block, 0, st>>>(a);
       else k_sweep_march<3, false, true, 0><<<grid, block, 0, st>>>(a);
     }
     GEM_LAUNCHED("k_sweep_march");
@@ -210,7 +245,7 @@ int launch_ghost_fill(const gem_grid* g, Blocks B, const double* vs1i, int lsp, 
                       cudaStream_t st) {
   const Dims& d = g->dev.d;
   const GridDev& G = g->dev;
-  const long long ncol = (long long)(d.lx2 + 4) * (d.lx3 + 4) * lsp;
+  const long long ncol = ghost_x1_items(d, G.flagper, lsp, fused);
   const long long nrow2 = (long long)(d.lx1 + 4) * (d.lx3 + 4) * lsp;
   const long long nrow3 = (long long)(d.lx1 + 4) * (d.lx2 + 4) * lsp;
   if (fused) {
@@ -466,6 +501,11 @@ int gem_grid_create(const gem_grid_desc* desc, gem_grid** out) {
   };
   const size_t n1 = (size_t)(lx1 + 1) * lx2 * lx3, n2 = (size_t)lx1 * (lx2 + 1) * lx3,
                n3 = (size_t)lx1 * lx2 * (lx3 + 1);
+  // the sweeps' shared range tests assume narrower reciprocals; others take the slow path
+  auto narrow = [&](double y) {
+    if (!(std::fabs(y) >= std::ldexp(1.0, -200) && std::fabs(y) <= std::ldexp(1.0, 200))) G.wide = 1;
+  };
+  G.wide = 0;
   const double* need[] = {desc->dx1, desc->dx1i, desc->dx2, desc->dx2i, desc->dx3, desc->dx3i,
                           desc->h1, desc->h2, desc->h3, desc->h1x1i, desc->h2x1i, desc->h3x1i,
                           desc->h1x2i, desc->h2x2i, desc->h3x2i, desc->h1x3i, desc->h2x3i, desc->h3x3i};
@@ -499,6 +539,19 @@ int gem_grid_create(const gem_grid_desc* desc, gem_grid** out) {
     cp(ydxs.data(), ydxs.size(), &L.ydxs);
     cp(dxi.data(), dxi.size(), &L.dxi);
     cp(ydxi.data(), ydxi.size(), &L.ydxi);
+    std::vector<double> row(8 * (size_t)(l + 2), 0.0);
+    for (int j = 0; j <= l + 1; ++j) {
+      double* r = row.data() + 8 * j;
+      r[0] = dx[j + 1];
+      r[1] = ydx[j + 1];
+      r[2] = dxs[j];
+      r[3] = ydxs[j];
+      r[4] = dx[j];
+      r[5] = j >= 2 ? dxi[j - 2] : 1.0;
+      r[6] = j >= 2 ? ydxi[j - 2] : 1.0;
+      if (l > 1) narrow(ydx[j]), narrow(ydx[j + 1]), narrow(ydxs[j]), narrow(r[6]);
+    }
+    cp(row.data(), row.size(), &L.row);
   }
   // Metric tables.  When no metric factor varies along x3 (checked bit for bit over the
   // interior x3 range, the only one the kernels read), one x3 slice is stored and the x3
@@ -541,6 +594,8 @@ int gem_grid_create(const gem_grid_desc* desc, gem_grid** out) {
           for (int i1 = 1; i1 <= lx1; ++i1) {
             const size_t k = (size_t)((i1 + 1) + s2 * (i2 + 1) + (inv ? 0 : s3 * (i3 + 1)));
             ok = ok && y_in_range(y0[k]) && y_in_range(y1[k]) && y_in_range(yh1[k]);
+            narrow(y0[k]);
+            narrow(y1[k]);
           }
       if (!ok) rc = set_err(GEM_EINVAL, "metric factors outside [2^-400, 2^400]");
     }
@@ -600,6 +655,7 @@ int gem_grid_create(const gem_grid_desc* desc, gem_grid** out) {
         p1[k] = f.ha[k] * f.ha[k] * f.hb[k];
         yhc[k] = 1.0 / hc[k];
         ok = ok && y_in_range(yhc[k]);
+        narrow(yhc[k]);
       }
       if (!ok) rc = set_err(GEM_EINVAL, "x%d face metric factors outside [2^-400, 2^400]", dd + 1);
       FaceTab& T = G.F[dd];
@@ -670,6 +726,7 @@ int gem_work_create(const gem_grid* g, gem_work** out) {
   w->acc = nullptr;
   w->Ttop = nullptr;
   w->lu = nullptr;
+  w->sweep = nullptr;
   w->sub = nullptr;
   std::memset(&w->src, 0, sizeof(w->src));
   w->has_src = 0;
@@ -716,7 +773,7 @@ int gem_work_destroy(gem_work* w) {
   for (cudaEvent_t e : w->ev)
     if (e) cudaEventDestroy(e);
   if (w->cs) cudaStreamDestroy(w->cs);
-  void* ps[] = {w->vs1i, w->vs2i, w->vs3i, w->nn, w->Tn, w->dt, w->acc, w->F, w->A, w->E, w->Ttop, w->lu, w->sub};
+  void* ps[] = {w->vs1i, w->vs2i, w->vs3i, w->nn, w->Tn, w->dt, w->acc, w->F, w->A, w->E, w->Ttop, w->lu, w->sweep, w->sub};
   for (void* p : ps)
     if (p) cudaFree(p);
   delete w;
@@ -800,7 +857,9 @@ int gem_work_prepare(gem_work* w, const gem_grid* g) {
   if (w->lx1 != g->dev.d.lx1 || w->lx2 != g->dev.d.lx2 || w->lx3 != g->dev.d.lx3)
     return set_err(GEM_EINVAL, "work object and grid sizes differ");
   double* p = nullptr;
-  return work_lu(w, g, &p);
+  SweepArgs a;
+  const int rc = work_lu(w, g, &p);
+  return rc ? rc : work_sweeps(w, g, a);
 }
 
 int gem_work_substep_buffers(gem_work* w, const gem_source_inputs** src, double** Q, double** Pr, double** Lo) {
@@ -1144,6 +1203,7 @@ static int fluid_adv_impl(const gem_cfg* cfg, const gem_grid* g, double* fluidva
   a.vs1i = w->vs1i;
   a.dtp = dt;
   a.which = 0;
+  if ((rc = work_sweeps(w, g, a))) return rc;
   if ((rc = launch_sweep(g, 3, true, a, LSP, st))) return rc;
   w->timer.record(3, st);
   if ((rc = launch_sweep(g, 1, true, a, LSP, st))) return rc;
@@ -1200,9 +1260,10 @@ static int advection_keepre(const gem_grid* g, double* fluidvars, double* fluida
   a.dtp = dt;
   a.dtp_w = nullptr;
   a.which = 0;
+  if ((rc = work_sweeps(w, g, a))) return rc;
   if ((rc = launch_sweep(g, 3, true, a, LSP, st))) return rc;
   if ((rc = launch_sweep(g, 1, true, a, LSP, st))) return rc;
-  const dim3 block(32, LSP), grid((d.lx1 + 31) / 32, d.lx3);
+  const dim3 block(32, LSP), grid((d.lx1 + 31) / 32, d.lx3, a.nsB ? sweep_parts(d, 2) : 1);
   if (g->dev.unit)
     k_sweep_march<2, true, true, 2, true><<<grid, block, 0, st>>>(a);
   else

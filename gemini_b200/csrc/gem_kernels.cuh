@@ -105,6 +105,9 @@ struct Line1D {
   const double *dx, *ydx;    // dx(j), j = 0..l+2, at [j]
   const double *dxs, *ydxs;  // dx(j) + dx(j+1), j = 0..l+1, at [j]
   const double *dxi, *ydxi;  // dxi(j), j = 1..l, at [j-1]
+  // the sweeps' row j = 0..l+1, 8 doubles: dx(j+1), 1/dx(j+1), dx(j)+dx(j+1) and its
+  // reciprocal, dx(j), dxi(j-1), 1/dxi(j-1) (1 outside 1..l), 0
+  const double* row;
 };
 
 // face tables of one sweep direction: ha2i for frank 0 and 1, the advected-direction metric
@@ -124,6 +127,7 @@ struct GridDev {
   const double *ha1_0, *ha1_1, *yha1_0, *yha1_1;  // h1*h2*h3, h1*h1*h2*h3 and reciprocals
   const double *dl[3], *ydl[3];                   // dx{d}i*h{d} per cell and reciprocals
   int dl3_tab;                                    // dl[2]/ydl[2] present (else formed in the kernel)
+  int wide;  // a tabulated reciprocal outside [2^-200, 2^200]: the sweeps' quotients test each numerator
   FaceTab F[3];
   const unsigned char* nullpts;
 };
@@ -177,12 +181,6 @@ __device__ __forceinline__ bool is_null(const GridDev& G, int i1, int i2, int i3
   return G.has_null && G.nullpts[ci(G.d, i1, i2, i3)];
 }
 
-// advec.f90:438-447
-__device__ __forceinline__ double minmod(double a, double b) {
-  if (a * b <= 0.0) return 0.0;
-  if (fabs(a) < fabs(b)) return a;
-  return b;
-}
 __device__ __forceinline__ double fmin_f(double a, double b) { return (a < b) ? a : b; }
 __device__ __forceinline__ double fmax_f(double a, double b) { return (a > b) ? a : b; }
 
@@ -202,7 +200,7 @@ struct Blocks {
 
 // v12rhov1 and T2rhoe on one value (multifluid.f90:193-214)
 __device__ __forceinline__ double conv_rv(double n, double v1, int s) { return n * c_ms[s] * v1; }
-__device__ __forceinline__ double conv_re(double n, double T, int s) { return n * KB * T / c_gm1[s]; }
+__device__ __forceinline__ double conv_re(double n, double T, int s) { return mdiv(n * KB * T, c_gm1[s], c_ygm1[s]); }
 
 // ======================================================================================
 // 2. Elementwise conversions over the full ghosted arrays (multifluid.f90:179-233)
@@ -387,13 +385,30 @@ struct GhostSrc {
 // own values, as the reference's full-slice assignments do.  In CONV mode the column's
 // interior momentum/energy values are also materialised for ghost columns (pass B/C read
 // them), interior columns keep them implicit.
+// work items of the pass: a thread per (column, species), and in CONV mode on periodic grids
+// one per interior x1 cell of the four x3-ghost planes
+__host__ __device__ __forceinline__ long long ghost_x1_items(const Dims& d, int flagper, int lsp, bool conv) {
+  const long long cols = (long long)(d.lx2 + 4) * (d.lx3 + 4) * lsp;
+  return cols + (conv && flagper ? 4LL * d.lx1 * d.lx2 * lsp : 0);
+}
 template <bool CONV>
 __device__ __forceinline__ void b_ghost_x1(const GridDev& G, const Blocks& B, const double* __restrict__ vs1i, int lsp, const VB vb) {
   const Dims d = G.d;
   const int n2 = d.lx2 + 4, n3 = d.lx3 + 4;
   const long long ncol = (long long)n2 * n3;
-  for (long long t = vb.bx * (long long)blockDim.x + threadIdx.x; t < ncol * lsp;
-       t += (long long)vb.gx * blockDim.x) {
+  const long long nend = ghost_x1_items(d, G.flagper, lsp, CONV);
+  for (long long t = vb.bx * (long long)blockDim.x + threadIdx.x; t < nend; t += (long long)vb.gx * blockDim.x) {
+    if (t >= ncol * lsp) {
+      // the interior x1 values of the periodic x3-ghost columns, a cell each: one thread per
+      // column walking x1 took 43 us at 96x32x32, this and the column threads 5
+      const long long q = t - ncol * lsp, row = q / d.lx1, pl = row / d.lx2;
+      const int i1 = (int)(q - row * d.lx1) + 1, i2 = (int)(row - pl * d.lx2) + 1, g = (int)(pl & 3);
+      const int s = (int)(pl >> 2);
+      const long long k = gi(d, i1, i2, (g < 2) ? g - 1 : d.lx3 + g - 1);
+      B.rv(s)[k] = GhostSrc::rv<true>(B, s, k);
+      B.re(s)[k] = GhostSrc::re<true>(B, s, k);
+      continue;
+    }
     const int s = (int)(t / ncol);
     const long long c = t - s * ncol;
     const int j2 = (int)(c % n2) - 1, j3 = (int)(c / n2) - 1;
@@ -409,13 +424,6 @@ __device__ __forceinline__ void b_ghost_x1(const GridDev& G, const Blocks& B, co
     const double msp = c_ms[s];
     const int lx1 = d.lx1;
     auto at = [&](int i1) { return gi(d, i1, j2, j3); };
-    if (!interior && CONV) {
-      for (int i1 = 1; i1 <= lx1; ++i1) {
-        const long long k = at(i1);
-        rvp[k] = GhostSrc::rv<true>(B, s, k);
-        rep[k] = GhostSrc::re<true>(B, s, k);
-      }
-    }
     // ---- bottom (advec.f90:42-60)
     {
       double n0, nm1, r0;
@@ -434,7 +442,7 @@ __device__ __forceinline__ void b_ghost_x1(const GridDev& G, const Blocks& B, co
       n[at(-1)] = nm1;
       rvp[at(-1)] = rm1 * nm1 * msp;
       rvp[at(0)] = r0 * n0 * msp;
-      const double e1 = interior ? GhostSrc::re<CONV>(B, s, at(1)) : rep[at(1)];
+      const double e1 = GhostSrc::re<CONV>(B, s, at(1));
       const double Tb = e1 / n[at(1)];
       rep[at(0)] = Tb * n0;
       rep[at(-1)] = Tb * nm1;
@@ -457,7 +465,7 @@ __device__ __forceinline__ void b_ghost_x1(const GridDev& G, const Blocks& B, co
       n[at(lx1 + 2)] = n2v;
       rvp[at(lx1 + 1)] = r1 * n1 * msp;
       rvp[at(lx1 + 2)] = r2 * n2v * msp;
-      const double el = interior ? GhostSrc::re<CONV>(B, s, at(lx1)) : rep[at(lx1)];
+      const double el = GhostSrc::re<CONV>(B, s, at(lx1));
       const double Tb = el / n[at(lx1)];
       rep[at(lx1 + 1)] = Tb * n1;
       rep[at(lx1 + 2)] = Tb * n2v;
@@ -681,48 +689,113 @@ struct SweepArgs {
   const double* dtp;
   double* dtp_w;  // writable alias of dtp (batched dt finalize); unused by the sweeps
   int which;      // standalone field set
+  // fused sweeps out of place (all null: in place): the densities between x3 and x2, and the
+  // momentum and energy densities between x1 and x2, in blocks of the state blocks' layout
+  double *nsB = nullptr, *rvB = nullptr, *reB = nullptr;
 };
 
-// Running state of one field while marching j = 0..lx+1 along a line:
-//   fp = f(j-1), fc = f(j), ls = lslope, slp = slope(j-1), php = phi(j-1)
-struct FieldRun {
-  double fp, fc, ls, slp, php;
-};
+// ---- the scheme of one field at one position -----------------------------------------------
+// The quotients of a position share range tests instead of testing each numerator (mdiv):
+//  - every field value of the line so far is 0 or in [2^-480, 2^480], so the slopes'
+//    numerators (differences of two of them) are 0 or at least 2^-533;
+//  - the update's first numerator dt*(Pr - Pl) is 0 or in [2^-500, 2^500], so its quotient by
+//    dxi, the second numerator, is 0 or in [2^-700, 2^700];
+//  - the face velocity is 0 or in [2^-500, 2^500];
+//  - every tabulated reciprocal is in [2^-200, 2^200] (GridDev::wide is 0).
+// Then no quotient or remainder over- or underflows and each equals the IEEE quotient, as in
+// mdiv; a zero numerator keeps its sign because the remainder is formed negated (b*q0 - a).
+// Anything else repeats the position with mdiv.  Thirteen branches a position (an ion's three
+// fields) become four, and the code between them is long enough to interleave.  With it, 32-bit
+// line offsets, one packed row of 1-D tables a position and x3-invariant metrics read once a
+// line, at 384x192x192: x3 2.81 -> 2.26 ms, x2 3.46 -> 3.23 (issue 49%, FP64 pipe 20%, DRAM
+// under 20% of peak: bound by the instruction count and fixed latencies at 14 warps per SM).
+__device__ __forceinline__ double fdiv(double a, double b, double y) {
+  const double q0 = a * y;
+  return __fma_rn(-__fma_rn(q0, b, -a), y, q0);
+}
+__device__ __forceinline__ bool in_range(double a, unsigned lo, unsigned span) {
+  const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  return (h - (lo << 20) < (span << 20)) | ((h | (unsigned)__double2loint(a)) == 0u);
+}
+__device__ __forceinline__ bool field_ok(double f) { return in_range(f, 543u, 960u); }
+__device__ __forceinline__ bool num_ok(double a) { return in_range(a, 523u, 1000u); }
 
-// Face quantities shared by the fields of one species at face j:
-//   v = v1i(j), hv = 0.5*v, qp = dx(j) + v/h1i(j)*dt, qm = dx(j) - v/h1i(j)*dt
+// Row j of a line's 1-D tables (Line1D::row).
+struct LineRow {
+  double dxn, ydxn, dxs, ydxs, dx, dxi, ydxi;
+};
+__device__ __forceinline__ LineRow line_row(const double* t, int j) {
+  const double2* q = reinterpret_cast<const double2*>(t + 8 * j);
+  const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), e = __ldg(q + 3);
+  return LineRow{a.x, a.y, b.x, b.y, c.x, c.y, e.x};
+}
+
+// Face quantities shared by the fields of one species at face j: the velocity v, which side is
+// upwind (neg: v < 0, cell j), and the slope's factor 0.5*v*(dx(j) -+ v/h1i(j)*dt), its sign
+// included (advec.f90:418-424; adding the negated product is the same as subtracting it).
 struct Face {
-  double v, hv, qp, qm;
+  double v, c;
+  bool neg;
 };
-
+template <bool UNIT>
 __device__ __forceinline__ Face make_face(double v, double hc, double yhc, double dxj, double dt) {
   Face f;
   f.v = v;
-  f.hv = 0.5 * v;
-  const double q = mdiv(v, hc, yhc) * dt;
-  f.qp = dxj + q;
-  f.qm = dxj - q;
+  f.neg = v < 0;
+  double q = UNIT ? v : fdiv(v, hc, yhc);
+  if (!UNIT && !num_ok(v)) q = slow_div(v, hc);
+  q = q * dt;
+  const double hv = 0.5 * v;
+  f.c = hv * (f.neg ? dxj + q : dxj - q);
+  if (f.neg) f.c = -f.c;
   return f;
 }
 
-// slope(j) (advec.f90:407-414): needs f(j-1), f(j), f(j+1) and lslope = rslope(j-1)
-__device__ __forceinline__ double mc_slope(double fm, double f0, double fpl, double ls, const Line1D& L,
-                                           int j, double& rs) {
-  rs = mdiv(fpl - f0, __ldg(L.dx + j + 1), __ldg(L.ydx + j + 1));
-  const double cs = mdiv(fpl - fm, __ldg(L.dxs + j), __ldg(L.ydxs + j));
-  return minmod(cs, minmod(2 * ls, 2 * rs));
+// slope(j) (advec.f90:407-414) from 2*lslope, 2*rslope and the centred slope:
+// minmod(cs, minmod(2*ls, 2*rs)) (minmod: advec.f90:438-447) with one select of zero for both
+__device__ __forceinline__ double mc_limit(double cs, double l2, double r2) {
+  const double m = (fabs(l2) < fabs(r2)) ? l2 : r2;
+  const bool zero = (l2 * r2 <= 0.0) | (cs * m <= 0.0);
+  const double t = (fabs(cs) < fabs(m)) ? cs : m;
+  return zero ? 0.0 : t;
 }
 
-// phi(j) (advec.f90:418-424)
+// flux phi(j) (advec.f90:418-424)
 __device__ __forceinline__ double mc_phi(double fjm1, double fj, double sljm1, double slj, const Face& F) {
-  if (F.v < 0) return fj * F.v - F.hv * F.qp * slj;
-  return fjm1 * F.v + F.hv * F.qm * sljm1;
+  return (F.neg ? fj : fjm1) * F.v + F.c * (F.neg ? slj : sljm1);
 }
 
-// updated cell value (advec.f90:427): f - dt*(Pr - Pl)/dxi/ha1 with P = ha2i*phi
-__device__ __forceinline__ double mc_update(double f, double Pr, double Pl, double dt, double dxi, double ydxi,
-                                            double ha1, double yha1) {
-  return f - mdiv(mdiv(dt * (Pr - Pl), dxi, ydxi), ha1, yha1);
+// Running state of one field while marching along a line:
+//   fp = f(j-1), fc = f(j), l2 = 2*lslope(j), slp = slope(j-1), P = ha2i*phi of face j-1
+struct FieldRun {
+  double fp, fc, l2, slp, P;
+};
+struct FieldOut {
+  double r2, sl, P, out;  // 2*rslope(j), slope(j), ha2i*phi of face j, updated cell j-1
+};
+// slope at j, flux through face j, update of cell j-1: f - dt*(Pr - Pl)/dxi/ha1 (advec.f90:427)
+template <bool UNIT>
+__device__ __forceinline__ FieldOut field_fast(const FieldRun& r, double fn, const LineRow& L, const Face& F, double ha2,
+                                               double dt, double ha1, double yha1, bool& ok) {
+  FieldOut o;
+  o.r2 = 2 * fdiv(fn - r.fc, L.dxn, L.ydxn);
+  o.sl = mc_limit(fdiv(fn - r.fp, L.dxs, L.ydxs), r.l2, o.r2);
+  const double ph = mc_phi(r.fp, r.fc, r.slp, o.sl, F);
+  o.P = UNIT ? ph : ha2 * ph;
+  const double a = dt * (o.P - r.P);
+  ok = ok & num_ok(a);
+  const double q = fdiv(a, L.dxi, L.ydxi);
+  o.out = r.fp - (UNIT ? q : fdiv(q, ha1, yha1));
+  return o;
+}
+__device__ __forceinline__ FieldOut field_any(const FieldRun& r, double fn, const LineRow& L, const Face& F, double ha2, double dt, double ha1,
+                                           double yha1) {
+  FieldOut o;
+  o.r2 = 2 * mdiv(fn - r.fc, L.dxn, L.ydxn);
+  o.sl = mc_limit(mdiv(fn - r.fp, L.dxs, L.ydxs), r.l2, o.r2);
+  o.P = ha2 * mc_phi(r.fp, r.fc, r.slp, o.sl, F);
+  o.out = r.fp - mdiv(mdiv(dt * (o.P - r.P), L.dxi, L.ydxi), ha1, yha1);
+  return o;
 }
 
 template <bool UNIT>
@@ -762,8 +835,13 @@ __device__ __forceinline__ void cp_async_wait() {
 // KEEPRE (fused x2 only): the epilogue stops after rhov12v1 and clean_param(1), (2) and
 // stores the swept energy densities instead of converting them (rhoe2T and clean_param(3)
 // come after the compression sub-step).
-template <int DIM, bool UNIT, bool FUSED, int PERM = 2, bool KEEPRE = false>
-__device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
+// INV (x3 sweep, tabulated metrics that do not vary along x3): the line's metrics are read
+// once.
+// seg, nseg: this thread's part of the line; more than one part needs the fused sweeps'
+// separate inputs and outputs (SweepArgs::nsB ...), since a part's first cells are
+// neighbours of cells that another thread updates.
+template <int DIM, bool UNIT, bool FUSED, int PERM = 2, bool KEEPRE = false, bool INV = false>
+__device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb, int seg = 0, int nseg = 1) {
   const GridDev& G = P.G;
   const Dims d = G.d;
   const Blocks& B = P.B;
@@ -777,39 +855,71 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
   const bool valid = a <= d.lx1;
   const int aa = valid ? a : d.lx1;  // idle lanes read a valid line
   const int lx = (DIM == 3) ? d.lx3 : d.lx2;
-  const long long stride = (DIM == 3) ? d.s3 : d.s2;
-  const long long base = (DIM == 3) ? gi(d, aa, b, 0) - d.s3 : gi(d, aa, 0, b) - d.s2;
-  auto cell = [&](int j) -> long long { return base + (long long)(j + 1) * stride; };
-  auto cmet = [&](int j) -> long long { return (DIM == 3) ? cmi(G, aa, b, j) : cmi(G, aa, j, b); };
-  auto fmet = [&](int j) -> long long { return (DIM == 3) ? fmi(FT, aa, b, j) : fmi(FT, aa, j, b); };
-  auto fvel = [&](int j) -> long long {  // face j in the work arrays (full 3-D layout)
-    return (DIM == 3) ? f3i(d, aa, b, j) : f2i(d, aa, j, b);
-  };
+  const int len = (lx + nseg - 1) / nseg;
+  const int c0 = 1 + seg * len, c1 = min(lx, c0 + len - 1);  // the cells updated here
+  if (c0 > lx && lx > 1) return;
+  // line index j is off(j) doubles behind the line's first ghost; the offsets and the metric
+  // indices fit 32 bits (a block of that many doubles would not fit the device)
+  const unsigned st = (unsigned)((DIM == 3) ? d.s3 : d.s2);
+  const long long base = (DIM == 3) ? gi(d, aa, b, -1) : gi(d, aa, -1, b);
+  auto off = [&](int j) -> unsigned { return (unsigned)(j + 1) * st; };
+  const unsigned cst = (DIM == 3) ? (unsigned)G.c3 : (unsigned)d.s2;
+  const unsigned cm0 = (unsigned)((DIM == 3) ? cmi(G, aa, b, -1) : cmi(G, aa, -1, b));
+  auto cmet = [&](int j) -> unsigned { return cm0 + (unsigned)(j + 1) * cst; };
+  const unsigned fst = (DIM == 3) ? (unsigned)FT.t3 : (unsigned)FT.t2;
+  const unsigned fm0 = (unsigned)((DIM == 3) ? fmi(FT, aa, b, 1) : fmi(FT, aa, 1, b));
+  auto fmet = [&](int j) -> unsigned { return fm0 + (unsigned)(j - 1) * fst; };
 
-  int nf;
-  double* fld[3];
-  int frank[3];
-  if (FUSED) {
-    if (s < LSP - 1) {
-      nf = 3;
-      fld[0] = B.ns(s); fld[1] = B.rv(s); fld[2] = B.re(s);
-      frank[0] = 0; frank[1] = 1; frank[2] = 0;
+  const bool ion = s < LSP - 1;
+  const int nf = FUSED ? (ion ? 3 : 1) : 1;
+  // src: the fields (fused x3: ns, vs1, Ts), the velocities; dst: the swept fields
+  const double *src[3], *vel;
+  double* dst[3];
+  bool fr1;  // the second field (fused) or the field (standalone) has frank 1
+  if constexpr (FUSED) {
+    fr1 = ion;
+    const long long so = (long long)s * d.ng;
+    double* nsB = P.nsB ? P.nsB + so : B.ns(s);
+    if constexpr (DIM == 3) {
+      src[0] = B.ns(s) + base;
+      src[1] = B.vs1(s) + base;
+      src[2] = B.Ts(s) + base;
+      vel = B.vs3(s) + base;
+      dst[0] = ion ? nsB + base : B.re(s) + base;
+      dst[1] = B.rv(s) + base;
+      dst[2] = B.re(s) + base;
     } else {
-      nf = 1;
-      fld[0] = B.re(s); fld[1] = fld[0]; fld[2] = fld[0];
-      frank[0] = 0; frank[1] = 0; frank[2] = 0;
+      const double* re = P.reB ? P.reB + so : B.re(s);
+      src[0] = (ion ? nsB : re) + base;
+      src[1] = (P.rvB ? P.rvB + so : B.rv(s)) + base;
+      src[2] = re + base;
+      vel = B.vs2(s) + base;
+      dst[0] = B.ns(s) + base;
+      dst[1] = B.rv(s) + base;
+      dst[2] = (KEEPRE ? B.re(s) : B.Ts(s)) + base;
     }
   } else {
-    nf = 1;
-    fld[0] = (P.which == 0) ? B.ns(s) : (P.which == 1) ? B.rv(s) : B.re(s);
-    fld[1] = fld[0]; fld[2] = fld[0];
-    frank[0] = (P.which == 1) ? 1 : 0; frank[1] = frank[0]; frank[2] = frank[0];
+    fr1 = P.which == 1;
+    dst[0] = ((P.which == 0) ? B.ns(s) : (P.which == 1) ? B.rv(s) : B.re(s)) + base;
+    dst[1] = dst[2] = dst[0];
+    src[0] = src[1] = src[2] = dst[0];
+    // face j in the work arrays (full 3-D layout), at [(j-1)*vst]
+    vel = P.vsi + (long long)s * ((DIM == 3) ? nf3(d) : nf2(d)) + ((DIM == 3) ? f3i(d, aa, b, 1) : f2i(d, aa, 1, b));
   }
+  const unsigned vst = (DIM == 3) ? (unsigned)d.lx1 * (unsigned)d.lx2 : (unsigned)d.lx1;
   const bool per = (PERM == 2) ? (G.flagper != 0) : (PERM == 1);
   auto map3 = [&](int j) -> int {  // x3 ghosts after set_global_boundaries / the self-wrap
     if (j >= 1 && j <= lx) return j;
     if (per) return (j < 1) ? j + lx : j - lx;
     return (j < 1) ? 1 : lx;
+  };
+  // the x2 ghost rows are read from the state blocks, which hold them
+  auto ghost2 = [&](int f) -> const double* {
+    if constexpr (FUSED && DIM == 2) {
+      if (f == 0) return (ion ? B.ns(s) : B.re(s)) + base;
+      return (f == 1 ? B.rv(s) : B.re(s)) + base;
+    }
+    return src[f];
   };
   // raw loads of line index j (FUSED x3 converts ns, vs1, Ts into the three fields)
   struct Raw {
@@ -818,19 +928,19 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
   auto load_raw = [&](int j) -> Raw {
     Raw r;
     if (FUSED && DIM == 3) {
-      const long long k = cell(map3(j));
-      r.x[0] = B.ns(s)[k];
-      r.x[1] = (s < LSP - 1) ? B.vs1(s)[k] : 0.0;
-      r.x[2] = B.Ts(s)[k];
+      const unsigned k = off(map3(j));
+      r.x[0] = src[0][k];
+      r.x[1] = ion ? src[1][k] : 0.0;
+      r.x[2] = src[2][k];
     } else {
 #pragma unroll
-      for (int f = 0; f < 3; ++f) r.x[f] = (f < nf) ? fld[f][cell(j)] : 0.0;
+      for (int f = 0; f < 3; ++f) r.x[f] = (f < nf) ? ((j < 1 || j > lx) ? ghost2(f) : src[f])[off(j)] : 0.0;
     }
     return r;
   };
   auto fields_of = [&](const Raw& r, double* out) {
     if (FUSED && DIM == 3) {
-      if (s < LSP - 1) {
+      if (ion) {
         out[0] = r.x[0];
         out[1] = conv_rv(r.x[0], r.x[1], s);
         out[2] = conv_re(r.x[0], r.x[2], s);
@@ -848,9 +958,10 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
     // advec1D_MC_curv passes a single-cell line through; the fused x3 sweep still
     // materialises the converted momentum/energy densities
     if (FUSED && DIM == 3 && valid) {
-      const long long k = cell(1);
-      B.rv(s)[k] = conv_rv(B.ns(s)[k], B.vs1(s)[k], s);
-      B.re(s)[k] = conv_re(B.ns(s)[k], B.Ts(s)[k], s);
+      const unsigned k = off(1);
+      if (P.nsB && ion) dst[0][k] = src[0][k];
+      dst[1][k] = conv_rv(src[0][k], src[1][k], s);
+      dst[2][k] = conv_re(src[0][k], src[2][k], s);
     }
     return;
   }
@@ -862,46 +973,49 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
     fields_of(load_raw(2), wrap2);
   }
   FieldRun run[3];
+  bool rok[3];  // every value of the line so far in the fast quotients' range
   {
     double fm1[3], f0[3];
-    fields_of(load_raw(-1), fm1);
-    fields_of(load_raw(0), f0);
-    const double dx0 = __ldg(L.dx);
+    fields_of(load_raw(c0 - 2), fm1);
+    fields_of(load_raw(c0 - 1), f0);
+    const double dx0 = __ldg(L.dx + c0 - 1);
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       run[f].fp = fm1[f];
       run[f].fc = f0[f];
-      run[f].ls = mdiv(f0[f] - fm1[f], dx0, __ldg(L.ydx));
+      run[f].l2 = 2 * mdiv(f0[f] - fm1[f], dx0, __ldg(L.ydx + c0 - 1));
       run[f].slp = 0.0;
-      run[f].php = 0.0;
+      run[f].P = 0.0;
+      rok[f] = !G.wide && field_ok(fm1[f]) && field_ok(f0[f]);
     }
   }
-  double ha2prev0 = 0.0, ha2prev1 = 0.0;
   // prefetch pipeline: each warp stages, three steps ahead, the raw values of f(jj) and the
   // velocity of step jj-1 (fused: the cell velocity v(jj-1); unfused: the face velocity
   // of face jj-1) by cp.async into slot jj&3 of a 4-slot shared ring of its own; step j
-  // reads slot (j+1)&3.  The sweep writes cell j-1 in place at step j, behind every staged
+  // reads slot (j+1)&3.  In place, the sweep writes cell j-1 at step j, behind every staged
   // index (up to j+4).  vprev = v(j-1).
   double vprev = 0.0;
   __shared__ double xm_f[LSP][4][4][32];
   auto stage = [&](int jj) {
-    if (jj >= 1 && jj <= lx + 2) {
+    if (jj <= c1 + 2) {
       double* sl = &xm_f[s][jj & 3][0][threadIdx.x];
       if constexpr (FUSED && DIM == 3) {
-        const long long k = cell(map3(jj));
-        cp_async8(sl, B.ns(s) + k);
-        if (s < LSP - 1) cp_async8(sl + 32, B.vs1(s) + k);
-        cp_async8(sl + 64, B.Ts(s) + k);
-        cp_async8(sl + 96, B.vs3(s) + cell(map3(jj - 1)));
+        const unsigned k = off(map3(jj));
+        cp_async8(sl, src[0] + k);
+        if (ion) cp_async8(sl + 32, src[1] + k);
+        cp_async8(sl + 64, src[2] + k);
+        cp_async8(sl + 96, vel + off(map3(jj - 1)));
       } else {
+        const bool gh = jj > lx;
+        const unsigned k = off(jj);
 #pragma unroll
         for (int f = 0; f < 3; ++f)
-          if (f < nf) cp_async8(sl + 32 * f, fld[f] + cell(jj));
+          if (f < nf) cp_async8(sl + 32 * f, (gh ? ghost2(f) : src[f]) + k);
         if constexpr (FUSED) {
           const int jv = (jj - 1 < 1) ? 1 : (jj - 1 > lx ? lx : jj - 1);
-          cp_async8(sl + 96, B.vs2(s) + cell(jv));
+          cp_async8(sl + 96, vel + off(jv));
         } else if (jj >= 2) {
-          cp_async8(sl + 96, P.vsi + (long long)s * ((DIM == 3) ? nf3(d) : nf2(d)) + fvel(jj - 1));
+          cp_async8(sl + 96, vel + (unsigned)(jj - 2) * vst);
         }
       }
     }
@@ -911,49 +1025,67 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
   // steps ahead, into a 4-slot shared ring (cp.async; warp s copies table s, warp 0 also
   // table 7): step j reads slot j&3 -- face j's hc, yhc, ha2i0, ha2i1 and cell j-1's ha1,
   // yha1 for frank 0 and 1.  Every step ends in a block barrier (the epilogue's, or its
-  // own for j < 2), and a thread waits for its copies two steps old before it, so step j+3's
-  // slot is complete and visible when step j+3 starts, and the slot written during step j
-  // was last read during step j-1, before that step's barrier.
+  // own in the first two steps), and a thread waits for its copies two steps old before it,
+  // so step j+3's slot is complete and visible when step j+3 starts, and the slot written
+  // during step j was last read during step j-1, before that step's barrier.
   constexpr bool SMETA = FUSED && DIM == 2 && !UNIT;
   __shared__ double sh_m[SMETA ? 4 : 1][SMETA ? 8 : 1][32];
   auto meta_issue = [&](int jj) {
     if constexpr (SMETA) {
-      if (jj >= 1 && jj <= lx + 1) {
+      if (jj <= c1 + 1) {
         double* slot = &sh_m[jj & 3][0][0];
         auto one = [&](int t) {
-          const double* src;
+          const double* p;
           if (t < 4) {
-            const long long fk = fmet(jj);
-            src = (t == 0 ? FT.hc : t == 1 ? FT.yhc : t == 2 ? FT.ha2i0 : FT.ha2i1) + fk;
+            p = (t == 0 ? FT.hc : t == 1 ? FT.yhc : t == 2 ? FT.ha2i0 : FT.ha2i1) + fmet(jj);
           } else {
             if (jj < 2) return;
-            const long long ck = cmet(jj - 1);
-            src = (t == 4 ? G.ha1_0 : t == 5 ? G.yha1_0 : t == 6 ? G.ha1_1 : G.yha1_1) + ck;
+            p = (t == 4 ? G.ha1_0 : t == 5 ? G.yha1_0 : t == 6 ? G.ha1_1 : G.yha1_1) + cmet(jj - 1);
           }
-          cp_async8(slot + t * 32 + threadIdx.x, src);
+          cp_async8(slot + t * 32 + threadIdx.x, p);
         };
         one(s);
         if (s == 0) one(7);
       }
     }
   };
+  // the line's metrics: x3-invariant ones once, the others where they are used
+  double mhc = 1.0, myhc = 1.0, ha2_0 = 1.0, ha2_1 = 1.0, ha1_0 = 1.0, yha1_0 = 1.0, ha1_1 = 1.0, yha1_1 = 1.0;
+  auto face_metrics = [&](unsigned k) {
+    mhc = __ldg(FT.hc + k);
+    myhc = __ldg(FT.yhc + k);
+    ha2_0 = __ldg(FT.ha2i0 + k);
+    if (fr1) ha2_1 = __ldg(FT.ha2i1 + k);
+  };
+  auto cell_metrics = [&](unsigned k) {
+    ha1_0 = __ldg(G.ha1_0 + k);
+    yha1_0 = __ldg(G.yha1_0 + k);
+    if (fr1) {
+      ha1_1 = __ldg(G.ha1_1 + k);
+      yha1_1 = __ldg(G.yha1_1 + k);
+    }
+  };
+  if constexpr (INV && !UNIT) {
+    face_metrics(fmet(1));
+    cell_metrics(cmet(1));
+  }
   // one cp.async group per step: the group committed at step j holds the metrics of step
   // j+3 and the staged values of slot (j+4)&3 (read at step j+3); the prologue commits the
-  // groups that steps 0..2 read
-  meta_issue(1);
-  stage(1);
+  // groups that the first three steps read
+  meta_issue(c0);
+  stage(c0);
   cp_async_commit();
-  meta_issue(2);
-  stage(2);
+  meta_issue(c0 + 1);
+  stage(c0 + 1);
   cp_async_commit();
-  stage(3);
+  stage(c0 + 2);
   cp_async_commit();
   if constexpr (SMETA) {
     cp_async_wait<0>();
     __syncthreads();
   }
 
-  for (int j = 0; j <= lx + 1; ++j) {
+  for (int j = c0 - 1; j <= c1 + 1; ++j) {
     // values of this step
     double fn[3];
     double vc = 0.0;  // fused: v(j); unfused: the velocity of face j
@@ -965,22 +1097,22 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
       cp_async_wait<3>();  // this thread's copies of step j-3's group (slot (j+1)&3)
       __syncwarp();
       const double* sl = &xm_f[s][(j + 1) & 3][0][threadIdx.x];
-      if (FUSED && DIM == 3 && j + 1 > lx) {
+      if (FUSED && DIM == 3 && per && j + 1 > lx) {
 #pragma unroll
-        for (int f = 0; f < 3; ++f) fn[f] = per ? ((j + 1 == lx + 1) ? wrap1[f] : wrap2[f]) : run[f].fc;
+        for (int f = 0; f < 3; ++f) fn[f] = (j == lx) ? wrap1[f] : wrap2[f];
       } else {
         Raw nx;
         nx.x[0] = sl[0];
-        nx.x[1] = (FUSED && DIM == 3) ? ((s < LSP - 1) ? sl[32] : 0.0) : ((nf > 1) ? sl[32] : 0.0);
+        nx.x[1] = (nf > 1) ? sl[32] : 0.0;
         nx.x[2] = ((FUSED && DIM == 3) || nf > 2) ? sl[64] : 0.0;
         fields_of(nx, fn);
       }
       vc = sl[96];
     }
 
-    Face F = {0.0, 0.0, 0.0, 0.0};
-    double ha2j0 = 0.0, ha2j1 = 0.0;
-    if (j >= 1) {
+    const LineRow R = line_row(L.row, j);
+    Face F = {0.0, 0.0, false};
+    if (j >= c0) {
       double v;
       if (!FUSED) {
         v = vc;
@@ -988,81 +1120,73 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
         v = 0.5 * (vprev + vc);
         vprev = vc;
       }
-      const double dxc = __ldg(L.dx + j);
-      if (UNIT) {
-        F = make_face(v, 1.0, 1.0, dxc, dt);
-        ha2j0 = ha2j1 = 1.0;
-      } else if constexpr (SMETA) {
-        const double* m = &sh_m[j & 3][0][threadIdx.x];
-        F = make_face(v, m[0], m[32], dxc, dt);
-        ha2j0 = m[64];
-        ha2j1 = m[96];
+      if constexpr (UNIT) {
+        F = make_face<true>(v, 1.0, 1.0, R.dx, dt);
       } else {
-        const long long fk = fmet(j);
-        F = make_face(v, __ldg(FT.hc + fk), __ldg(FT.yhc + fk), dxc, dt);
-        ha2j0 = __ldg(FT.ha2i0 + fk);
-        ha2j1 = __ldg(FT.ha2i1 + fk);
+        if constexpr (SMETA) {
+          const double* m = &sh_m[j & 3][0][threadIdx.x];
+          mhc = m[0];
+          myhc = m[32];
+          ha2_0 = m[64];
+          ha2_1 = m[96];
+        } else if constexpr (!INV) {
+          face_metrics(fmet(j));
+        }
+        F = make_face<false>(v, mhc, myhc, R.dx, dt);
       }
     } else if (FUSED) {
       vprev = vc;
     }
-    double ha1_0 = 1.0, yha1_0 = 1.0, ha1_1 = 1.0, yha1_1 = 1.0, dxi = 0.0, ydxi = 0.0;
-    if (j >= 2) {
-      dxi = __ldg(L.dxi + j - 2);
-      ydxi = __ldg(L.ydxi + j - 2);
-      if constexpr (SMETA) {
+    if constexpr (SMETA) {
+      if (j > c0) {
         const double* m = &sh_m[j & 3][4][threadIdx.x];
         ha1_0 = m[0];
         yha1_0 = m[32];
-        if (frank[0] == 1 || frank[1] == 1) {
+        if (fr1) {
           ha1_1 = m[64];
           yha1_1 = m[96];
         }
-      } else {
-        const long long ck = cmet(j - 1);
-        cell_metric<UNIT>(G, ck, 0, ha1_0, yha1_0);
-        if (frank[0] == 1 || frank[1] == 1) cell_metric<UNIT>(G, ck, 1, ha1_1, yha1_1);
       }
+    } else if constexpr (!UNIT && !INV) {
+      if (j > c0) cell_metrics(cmet(j - 1));
     }
+    // the first two positions of a line only fill the running state: their face (v = 0) or
+    // update is not used
     double outv[3];
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       if (f < nf) {
         FieldRun& r = run[f];
-        double rs;
-        const double sl = mc_slope(r.fp, r.fc, fn[f], r.ls, L, j, rs);
-        r.ls = rs;
-        if (j >= 1) {
-          const double ph = mc_phi(r.fp, r.fc, r.slp, sl, F);
-          const bool fr = frank[f] == 1;
-          if (j >= 2)
-            outv[f] = mc_update(r.fp, (fr ? ha2j1 : ha2j0) * ph, (fr ? ha2prev1 : ha2prev0) * r.php, dt, dxi, ydxi,
-                                fr ? ha1_1 : ha1_0, fr ? yha1_1 : yha1_0);
-          r.php = ph;
-        }
-        r.slp = sl;
+        const bool fr = FUSED ? f == 1 : fr1;
+        const double h2 = fr ? ha2_1 : ha2_0, h1 = fr ? ha1_1 : ha1_0, y1 = fr ? yha1_1 : yha1_0;
+        rok[f] = rok[f] & field_ok(fn[f]);
+        bool ok = rok[f];
+        FieldOut o = field_fast<UNIT>(r, fn[f], R, F, h2, dt, h1, y1, ok);
+        if (!ok) o = field_any(r, fn[f], R, F, h2, dt, h1, y1);
+        outv[f] = o.out;
+        r.l2 = o.r2;
+        r.P = o.P;
+        r.slp = o.sl;
         r.fp = r.fc;
         r.fc = fn[f];
       }
     }
-    ha2prev0 = ha2j0;
-    ha2prev1 = ha2j1;
     if constexpr (SMETA) {
-      if (j < 2) {
+      if (j <= c0) {
         cp_async_wait<2>();
         __syncthreads();
       }
     }
-    if (j < 2) continue;
+    if (j <= c0) continue;
     const int c = j - 1;  // finished cell
-    const long long kc = cell(c);
+    const unsigned kc = off(c);
     if constexpr (!(FUSED && DIM == 2)) {
       if (valid) {
 #pragma unroll
         for (int f = 0; f < 3; ++f)
-          if (f < nf) fld[f][kc] = outv[f];
-        if (FUSED && DIM == 3 && s == LSP - 1)  // unswept electron momentum density
-          B.rv(s)[kc] = conv_rv(B.ns(s)[kc], B.vs1(s)[kc], s);
+          if (f < nf) dst[f][kc] = outv[f];
+        if (FUSED && DIM == 3 && !ion)  // unswept electron momentum density
+          dst[1][kc] = conv_rv(src[0][kc], src[1][kc], s);
       }
     } else {
       // ---- fused x2 epilogue: rhov12v1 (multifluid.f90:218-233), clean_param(1),
@@ -1081,19 +1205,19 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
         if (nul) nc = (s == 0) ? MINDENSNULL * 1e-2 : MINDENSNULL;
         if constexpr (KEEPRE) {
           if (valid) {
-            B.ns(s)[kc] = nc;
-            B.rv(s)[kc] = r;
-            B.vs1(s)[kc] = nul ? 0.0 : v;
-            B.re(s)[kc] = e;
+            dst[0][kc] = nc;
+            dst[1][kc] = r;
+            (dst[0] + LSP * d.ng)[kc] = nul ? 0.0 : v;
+            dst[2][kc] = e;
           }
         } else {
           double T = fmax_f(c_gm1kb[s] * e / fmax_f(nc, MINDENSDIV), 100.0);
           if (nul) T = 100;
           if (valid) {
-            B.ns(s)[kc] = nc;
-            B.rv(s)[kc] = r;
-            B.vs1(s)[kc] = nul ? 0.0 : v;
-            B.Ts(s)[kc] = T;
+            dst[0][kc] = nc;
+            dst[1][kc] = r;
+            (dst[0] + LSP * d.ng)[kc] = nul ? 0.0 : v;
+            dst[2][kc] = T;
           }
         }
       }
@@ -1112,17 +1236,17 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
         const double ne = nul ? MINDENSNULL : npost;
         if constexpr (KEEPRE) {
           if (valid) {
-            B.ns(s)[kc] = ne;
-            B.vs1(s)[kc] = nul ? 0.0 : ve;
-            B.re(s)[kc] = outv[0];
+            dst[0][kc] = ne;
+            (dst[0] + LSP * d.ng)[kc] = nul ? 0.0 : ve;
+            dst[2][kc] = outv[0];
           }
         } else {
           double T = fmax_f(c_gm1kb[s] * outv[0] / fmax_f(ne, MINDENSDIV), 100.0);
           if (nul) T = 100;
           if (valid) {
-            B.ns(s)[kc] = ne;
-            B.vs1(s)[kc] = nul ? 0.0 : ve;
-            B.Ts(s)[kc] = T;
+            dst[0][kc] = ne;
+            (dst[0] + LSP * d.ng)[kc] = nul ? 0.0 : ve;
+            dst[2][kc] = T;
           }
         }
       }
@@ -1136,12 +1260,11 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb) {
 #ifndef GEM_MARCH_MINB
 #define GEM_MARCH_MINB 2
 #endif
-#ifndef GEM_X1_MINB
-#define GEM_X1_MINB 3
-#endif
-template <int DIM, bool UNIT, bool FUSED, int PERM = 2, bool KEEPRE = false>
+// blockIdx.z: the part of the line
+template <int DIM, bool UNIT, bool FUSED, int PERM = 2, bool KEEPRE = false, bool INV = false>
 __global__ void __launch_bounds__(224, GEM_MARCH_MINB) k_sweep_march(SweepArgs P) {
-  b_sweep_march<DIM, UNIT, FUSED, PERM, KEEPRE>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
+  b_sweep_march<DIM, UNIT, FUSED, PERM, KEEPRE, INV>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x},
+                                                     (int)blockIdx.z, (int)gridDim.z);
 }
 
 
@@ -1150,7 +1273,9 @@ __global__ void __launch_bounds__(224, GEM_MARCH_MINB) k_sweep_march(SweepArgs P
 // p = 0 .. lx1+1: the slope at cell p, the flux P(p) = ha2i(p)*phi(p) at face p, and the update
 // of cell p-1 (which needs P(p) and P(p-1)).  Values crossing the chunk edge (slope(p-1),
 // P(p-1)) are carried from lane 31 of the previous chunk.
-template <bool UNIT, bool FUSED>
+// OOP: out of place (SweepArgs::nsB ...); a template flag because the second set of pointers
+// costs registers that the in-place sweep of large grids does not have.
+template <bool UNIT, bool FUSED, bool OOP = false>
 __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
   const GridDev& G = P.G;
   const Dims d = G.d;
@@ -1163,20 +1288,27 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
   const Line1D& L = G.L[0];
   const FaceTab& FT = G.F[0];
   const long long col = gi(d, 0, i2, i3);  // cell i at col + i
-  int nf;
-  double* fld[3];
-  if (FUSED) {
-    if (s < LSP - 1) {
-      nf = 3;
-      fld[0] = B.ns(s); fld[1] = B.rv(s); fld[2] = B.re(s);
-    } else {
-      nf = 1;
-      fld[0] = B.re(s); fld[1] = fld[0]; fld[2] = fld[0];
-    }
+  // fld: the fields' column at cell 0; out of place, src / dst where they are read and written
+  // (the densities' x1 ghosts and the wrapped copies below stay in the state blocks)
+  const bool ion = s < LSP - 1;
+  const int nf = (FUSED && ion) ? 3 : 1;
+  double *fld[3], *src[3], *dst[3];
+  if constexpr (FUSED) {
+    fld[0] = (ion ? B.ns(s) : B.re(s)) + col;
+    fld[1] = B.rv(s) + col;
+    fld[2] = B.re(s) + col;
   } else {
-    nf = 1;
-    fld[0] = (P.which == 0) ? B.ns(s) : (P.which == 1) ? B.rv(s) : B.re(s);
-    fld[1] = fld[0]; fld[2] = fld[0];
+    fld[0] = ((P.which == 0) ? B.ns(s) : (P.which == 1) ? B.rv(s) : B.re(s)) + col;
+    fld[1] = fld[2] = fld[0];
+  }
+#pragma unroll
+  for (int f = 0; f < 3; ++f) src[f] = dst[f] = fld[f];
+  if constexpr (OOP) {
+    const long long so = (long long)s * d.ng + col;
+    if (ion) src[0] = P.nsB + so;
+    dst[0] = ion ? src[0] : P.reB + so;
+    dst[1] = P.rvB + so;
+    dst[2] = P.reB + so;
   }
   const double* V1 = B.vs1(s) + col;
   // fused: velocities of the two boundary faces (advec.f90:170-196)
@@ -1211,7 +1343,7 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
           const int ef = (e <= n + 2) ? e : n + 2;
 #pragma unroll
           for (int f = 0; f < 3; ++f)
-            if (f < nf) cp_async8(&xs_f[s][slot][f][t], fld[f] + col + ef);
+            if (f < nf) cp_async8(&xs_f[s][slot][f][t], ((OOP && f == 0 && (ef < 1 || ef > n)) ? fld[f] : src[f]) + ef);
           if constexpr (FUSED) cp_async8(&xs_f[s][slot][3][t], V1 + ((e >= 1 && e <= n) ? e : 1));
         }
         if constexpr (!FUSED) {
@@ -1256,29 +1388,23 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
     } else {
       v = sf[3 * XW + lane];
     }
-    Face F = {0.0, 0.0, 0.0, 0.0};
+    const int pi = pc >= 2 ? pc - 2 : 0;
+    const LineRow R{__ldg(L.dx + pc + 1), __ldg(L.ydx + pc + 1), __ldg(L.dxs + pc), __ldg(L.ydxs + pc), __ldg(L.dx + pc),
+                    __ldg(L.dxi + pi), __ldg(L.ydxi + pi)};
+    Face F;
     double ha2 = 1.0;
-    const double dxc = __ldg(L.dx + pc), ydxc = __ldg(L.ydx + pc);
-    const double dxn = __ldg(L.dx + pc + 1), ydxn = __ldg(L.ydx + pc + 1);
-    const double dxs = __ldg(L.dxs + pc), ydxs = __ldg(L.ydxs + pc);
-    {
-      if (UNIT) {
-        F = make_face(v, 1.0, 1.0, dxc, dt);
-      } else {
-        F = make_face(v, sm[lane], sm[32 + lane], dxc, dt);
-        ha2 = sm[64 + lane];
-      }
+    if (UNIT) {
+      F = make_face<true>(v, 1.0, 1.0, R.dx, dt);
+    } else {
+      F = make_face<false>(v, sm[lane], sm[32 + lane], R.dx, dt);
+      ha2 = sm[64 + lane];
     }
     // cell p-1 metrics for the update
     const int q = pc - 1;  // updated cell
-    double ha1 = 1.0, yha1 = 1.0, dxi = 1.0, ydxi = 1.0;
-    if (q >= 1 && q <= n) {
-      dxi = __ldg(L.dxi + q - 1);
-      ydxi = __ldg(L.ydxi + q - 1);
-      if constexpr (!UNIT) {
-        ha1 = sm[96 + lane];
-        yha1 = sm[128 + lane];
-      }
+    double ha1 = 1.0, yha1 = 1.0;
+    if constexpr (!UNIT) {
+      ha1 = sm[96 + lane];
+      yha1 = sm[128 + lane];
     }
     double outv[3];
 #pragma unroll
@@ -1287,38 +1413,41 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
         const double fm = sf[f * XW + lane];
         const double f0 = sf[f * XW + lane + 1];
         const double fpl = sf[f * XW + lane + 2];
-        // slope(p) (advec.f90:407-414) with lslope = rslope(p-1) from the lane below
-        const double rs = mdiv(fpl - f0, dxn, ydxn);
-        double ls = __shfl_up_sync(0xffffffffu, rs, 1);
-        if (lane == 0) ls = mdiv(f0 - fm, dxc, ydxc);
-        const double cs = mdiv(fpl - fm, dxs, ydxs);
-        const double sl = minmod(cs, minmod(2 * ls, 2 * rs));
+        // slope(p) (advec.f90:407-414) with lslope = rslope(p-1) from the lane below.  Each
+        // quotient tests its own numerator here: a test shared through a warp vote, as the
+        // march kernels share theirs through the line, cost more registers than it saved
+        // (3.45 ms against 3.14 at 384x192x192)
+        const double r2 = 2 * mdiv(fpl - f0, R.dxn, R.ydxn);
+        double l2 = __shfl_up_sync(0xffffffffu, r2, 1);
+        if (lane == 0) l2 = 2 * mdiv(f0 - fm, R.dx, __ldg(L.ydx + pc));
+        const double cs = mdiv(fpl - fm, R.dxs, R.ydxs);
+        const double sl = mc_limit(cs, l2, r2);
         double slm = __shfl_up_sync(0xffffffffu, sl, 1);
         if (lane == 0) slm = carry_sl[f];
         const double ph = mc_phi(fm, f0, slm, sl, F);
-        const double Pp = ha2 * ph;
+        const double Pp = UNIT ? ph : ha2 * ph;
         double Pm = __shfl_up_sync(0xffffffffu, Pp, 1);
         if (lane == 0) Pm = carry_P[f];
-        outv[f] = mc_update(fm, Pp, Pm, dt, dxi, ydxi, ha1, yha1);
+        const double dq = mdiv(dt * (Pp - Pm), R.dxi, R.ydxi);
+        outv[f] = fm - (UNIT ? dq : mdiv(dq, ha1, yha1));
         carry_sl[f] = __shfl_sync(0xffffffffu, sl, 31);
         carry_P[f] = __shfl_sync(0xffffffffu, Pp, 31);
       }
     }
     if (act && q >= 1 && q <= n) {
-      const long long kq = col + q;
 #pragma unroll
       for (int f = 0; f < 3; ++f)
-        if (f < nf) fld[f][kq] = outv[f];
+        if (f < nf) dst[f][q] = outv[f];
       if (FUSED && G.flagper) {
         // halo_allparams self-wrap of the updated column (mpihalo.f90:147-151)
         if (i3 >= d.lx3 - 1) {
-          const long long kw = gi(d, q, i2, i3 - d.lx3);
+          const long long kw = q - (long long)d.lx3 * d.s3;
 #pragma unroll
           for (int f = 0; f < 3; ++f)
             if (f < nf) fld[f][kw] = outv[f];
         }
         if (i3 <= 2) {
-          const long long kw = gi(d, q, i2, i3 + d.lx3);
+          const long long kw = q + (long long)d.lx3 * d.s3;
 #pragma unroll
           for (int f = 0; f < 3; ++f)
             if (f < nf) fld[f][kw] = outv[f];
@@ -1330,9 +1459,9 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
   cp_async_wait<0>();  // nothing in flight when the next work item (batched path) restages
 }
 
-template <bool UNIT, bool FUSED>
-__global__ void __launch_bounds__(224, GEM_X1_MINB) k_sweep_x1(SweepArgs P) {
-  b_sweep_x1<UNIT, FUSED>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
+template <bool UNIT, bool FUSED, bool OOP = false>
+__global__ void __launch_bounds__(224, OOP ? 2 : 3) k_sweep_x1(SweepArgs P) {
+  b_sweep_x1<UNIT, FUSED, OOP>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
 
