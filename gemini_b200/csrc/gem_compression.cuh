@@ -47,6 +47,13 @@ GEMC_HD double hm(const double* h, const View& v, int i1, int i2, int i3) {
 GEMC_HD long long ncell(const View& v) { return (long long)v.lx1 * v.lx2 * v.lx3; }
 // interior cell c (column-major 1:lx1,1:lx2,1:lx3) -> indices
 GEMC_HD void cell_of(const View& v, long long c, int& i1, int& i2, int& i3) {
+  if ((unsigned long long)c <= 0xffffffffull) {  // 32-bit quotients where the index fits
+    const unsigned u = (unsigned)c, r = u / (unsigned)v.lx1, q = r / (unsigned)v.lx2;
+    i1 = (int)(u - r * (unsigned)v.lx1) + 1;
+    i2 = (int)(r - q * (unsigned)v.lx2) + 1;
+    i3 = (int)q + 1;
+    return;
+  }
   i1 = (int)(c % v.lx1) + 1;
   const long long r = c / v.lx1;
   i2 = (int)(r % v.lx2) + 1;

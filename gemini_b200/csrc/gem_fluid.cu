@@ -1006,6 +1006,18 @@ int gem_clean_param_dev(const gem_grid* g, int iparm, double* fluidvars, void* s
   return GEM_OK;
 }
 
+// clean_param(3), (2), (1) in the order the source sub-step ends with
+static int clean_all(const gem_grid* g, double* fluidvars, cudaStream_t st) {
+  k_clean_all<<<grid_for(g->dev.d.ng, 256), 256, 0, st>>>(g->dev, blocks(g, fluidvars, nullptr));
+  GEM_LAUNCHED("k_clean_all");
+  if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
+    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * LSP;
+    k_clean_vel_edges<<<grid_for(n, 128), 128, 0, st>>>(g->dev, fluidvars + LSP * g->dev.d.ng);
+    GEM_LAUNCHED("k_clean_vel_edges");
+  }
+  return GEM_OK;
+}
+
 int gem_energy_diffusion_dev(const gem_cfg* cfg, const gem_grid* g, double* fluidvars,
                              const double* electrovars, const gem_work* w, const double* dt, void* stream) {
   if (!cfg || check_grid(g) || !fluidvars || !electrovars || !w || !dt) return set_err(GEM_EINVAL, "null argument");

@@ -40,12 +40,23 @@ int gem_fluid_adv_compression_dev(const gem_cfg* cfg, const gem_grid* g, double*
     GEM_TRY(gem_clean_param_dev(g, 2, fluidvars, stream));
   }
   // compression (app/main.f90:320-338)
-  GEM_TRY(gem_vnricht_artvisc_dev(g, fluidvars, Q, stream));
-  GEM_TRY(gem_halo_fluidvars_dev(g, fluidvars, fluidauxvars, stream));
-  GEM_TRY(gem_rk2_global_boundary_allspec_dev(g, fluidvars, stream));
-  GEM_TRY(gem_compression_dev(g, fluidvars, fluidauxvars, Q, dt, stream));
-  GEM_TRY(gem_rhoe2T_dev(g, fluidvars, fluidauxvars, stream));
-  GEM_TRY(gem_clean_param_dev(g, 3, fluidvars, stream));
+  if (d.lx1 >= 4 && !(g->dev.flagper && d.lx3 < 2)) {
+    // one pass over the interior cells, then the ghost velocities
+    const dim3 grid(grid_for(nci(d), 256), LSP);
+    const Blocks B = blocks(g, fluidvars, fluidauxvars);
+    if (g->dev.unit) gemk::kc_compress_T<true><<<grid, 256, 0, S(stream)>>>(g->dev, B, Q, dt);
+    else gemk::kc_compress_T<false><<<grid, 256, 0, S(stream)>>>(g->dev, B, Q, dt);
+    GEM_LAUNCHED("kc_compress_T");
+    GEM_TRY(gem_halo_fluidvars_dev(g, fluidvars, fluidauxvars, stream));
+    GEM_TRY(gem_rk2_global_boundary_allspec_dev(g, fluidvars, stream));
+  } else {
+    GEM_TRY(gem_vnricht_artvisc_dev(g, fluidvars, Q, stream));
+    GEM_TRY(gem_halo_fluidvars_dev(g, fluidvars, fluidauxvars, stream));
+    GEM_TRY(gem_rk2_global_boundary_allspec_dev(g, fluidvars, stream));
+    GEM_TRY(gem_compression_dev(g, fluidvars, fluidauxvars, Q, dt, stream));
+    GEM_TRY(gem_rhoe2T_dev(g, fluidvars, fluidauxvars, stream));
+    GEM_TRY(gem_clean_param_dev(g, 3, fluidvars, stream));
+  }
   // diffusion (app/main.f90:339-355)
   if (d.lx1 >= 4) {  // the diffusion store with clean_param(3) and T2rhoe folded in (the same results)
     GEM_TRY(diffusion_clean_T2rhoe(cfg, g, fluidvars, fluidauxvars, electrovars, w, dt, S(stream)));
@@ -70,10 +81,7 @@ int gem_source_loss_allparams_dev(const gem_grid* g, double* fluidvars, double* 
   GEM_TRY(gem_momentum_source_loss_solve_dev(g, dt, Pr, Lo, fluidvars, fluidauxvars, stream));
   GEM_TRY(gem_srcs_continuity_dev(g, in->nn, in->vn1, in->vn2, in->vn3, in->Tn, fluidvars, Pr, Lo, stream));
   GEM_TRY(gem_mass_source_loss_solve_dev(g, dt, Pr, Lo, in->Prionize, fluidvars, stream));
-  GEM_TRY(gem_clean_param_dev(g, 3, fluidvars, stream));
-  GEM_TRY(gem_clean_param_dev(g, 2, fluidvars, stream));
-  GEM_TRY(gem_clean_param_dev(g, 1, fluidvars, stream));
-  return GEM_OK;
+  return clean_all(g, fluidvars, S(stream));
 }
 
 long long gem_fluid_adv_full_scratch_doubles(const gem_grid* g) {

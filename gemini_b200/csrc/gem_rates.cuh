@@ -53,6 +53,7 @@ struct View {
   double pi;  // 4 atan(1), formed on the host
   // device only: RN(1/(ms_i + mn_j)) and RN(1/(ms_i + ms_j)), formed on the host (qdk)
   double ymn[NSP][NNEU], yms[NSP][NSP];
+  double mred[NSP][NSP], ymred[NSP][NSP];  // device only: ms_i ms_j / (ms_i + ms_j) and its RN reciprocal
 };
 
 GEMR_HD long long ncell(const View& v) { return (long long)v.lx1 * v.lx2 * v.lx3; }
@@ -62,7 +63,16 @@ GEMR_HD long long gix(const View& v, int i1, int i2, int i3) {
 GEMR_HD double hm(const double* h, const View& v, int i1, int i2, int i3) {
   return h ? h[(long long)(i1 + 1) + v.s2 * (i2 + 1) + v.c3 * (i3 + 1)] : 1.0;
 }
+// 32-bit quotients where the index fits (a 64-bit one costs about four times as many
+// instructions, and two a cell were a fifth of the rate kernels)
 GEMR_HD void cell_of(const View& v, long long c, int& i1, int& i2, int& i3) {
+  if ((unsigned long long)c <= 0xffffffffull) {
+    const unsigned u = (unsigned)c, r = u / (unsigned)v.lx1, q = r / (unsigned)v.lx2;
+    i1 = (int)(u - r * (unsigned)v.lx1) + 1;
+    i2 = (int)(r - q * (unsigned)v.lx2) + 1;
+    i3 = (int)q + 1;
+    return;
+  }
   i1 = (int)(c % v.lx1) + 1;
   const long long r = c / v.lx1;
   i2 = (int)(r % v.lx2) + 1;
@@ -77,22 +87,22 @@ GEMR_HD double p4(double x) {
 }
 
 // collisions.f90:12-55 coefficient tables (rows: charged species; columns: O, N2, O2, H or
-// the charged species), default-REAL literals; constant memory on the device
+// the charged species), default-REAL literals widened to double; constant memory on the device
 #ifdef __CUDACC__
 #define GEMR_TABLE __constant__ const
 #else
 #define GEMR_TABLE static const
 #endif
-GEMR_TABLE float kCsn[NSP][NNEU] = {{-1, 6.82e-10f, 6.64e-10f, -1},          {2.44e-10f, 4.34e-10f, 4.27e-10f, 0.69e-10f},
+GEMR_TABLE double kCsn[NSP][NNEU] = {{-1, 6.82e-10f, 6.64e-10f, -1},          {2.44e-10f, 4.34e-10f, 4.27e-10f, 0.69e-10f},
                                     {2.58e-10f, -1, 4.49e-10f, 0.74e-10f},    {2.31e-10f, 4.13e-10f, -1, 0.65e-10f},
                                     {4.42e-10f, 7.47e-10f, 7.25e-10f, 1.45e-10f}, {-1, 33.6e-10f, 32.0e-10f, -1},
                                     {-1, -1, -1, -1}};
-GEMR_TABLE float kC2sn1[NSP][NNEU] = {{3.67e-11f, 0, 0, 4.63e-12f}, {0, 0, 0, 0}, {0, 5.14e-11f, 0, 0},
+GEMR_TABLE double kC2sn1[NSP][NNEU] = {{3.67e-11f, 0, 0, 4.63e-12f}, {0, 0, 0, 0}, {0, 5.14e-11f, 0, 0},
                                       {0, 0, 2.59e-11f, 0},         {0, 0, 0, 0}, {6.61e-11f, 0, 0, 2.65e-10f},
                                       {-1, -1, -1, -1}};
-GEMR_TABLE float kC2sn2[NSP][NNEU] = {{0.064f, 0, 0, -1}, {0, 0, 0, 0},           {0, 0.069f, 0, 0}, {0, 0, 0.073f, 0},
+GEMR_TABLE double kC2sn2[NSP][NNEU] = {{0.064f, 0, 0, -1}, {0, 0, 0, 0},           {0, 0.069f, 0, 0}, {0, 0, 0.073f, 0},
                                       {0, 0, 0, 0},       {0.047f, 0, 0, 0.083f}, {-1, -1, -1, -1}};
-GEMR_TABLE float kCsj[NSP][NSP] = {{0.22f, 0.26f, 0.25f, 0.26f, 0.22f, 0.077f, 1.87e-3f},
+GEMR_TABLE double kCsj[NSP][NSP] = {{0.22f, 0.26f, 0.25f, 0.26f, 0.22f, 0.077f, 1.87e-3f},
                                    {0.14f, 0.16f, 0.16f, 0.17f, 0.13f, 0.042f, 9.97e-4f},
                                    {0.15f, 0.17f, 0.17f, 0.18f, 0.14f, 0.045f, 1.07e-3f},
                                    {0.13f, 0.16f, 0.15f, 0.16f, 0.12f, 0.039f, 9.347e-4f},
@@ -102,12 +112,16 @@ GEMR_TABLE float kCsj[NSP][NSP] = {{0.22f, 0.26f, 0.25f, 0.26f, 0.22f, 0.077f, 1
 GEMR_TABLE double kMn[NNEU] = {16, 28, 32, 1};  // neutral masses / amu, phys_consts.in.f90:41
 
 struct Coll {
-  static GEMR_HD double csn(int i, int j) { return (double)kCsn[i][j]; }
-  static GEMR_HD double c2sn1(int i, int j) { return (double)kC2sn1[i][j]; }
-  static GEMR_HD double c2sn2(int i, int j) { return (double)kC2sn2[i][j]; }
-  static GEMR_HD double csj(int i, int j) { return (double)kCsj[i][j]; }
+  static GEMR_HD double csn(int i, int j) { return kCsn[i][j]; }
+  static GEMR_HD double c2sn1(int i, int j) { return kC2sn1[i][j]; }
+  static GEMR_HD double c2sn2(int i, int j) { return kC2sn2[i][j]; }
+  static GEMR_HD double csj(int i, int j) { return kCsj[i][j]; }
   static GEMR_HD double mn(int j) { return kMn[j] * AMU_; }
 };
+
+#ifdef __CUDACC__
+__device__ __noinline__ double div_slow(double a, double b) { return a / b; }
+#endif
 
 // a/b for a constant divisor b whose correctly rounded reciprocal y = RN(1/b) was formed on
 // the host.  On the device: q0 = RN(a*y), the exact remainder a - b*q0 and RN(q0 + r*y),
@@ -121,7 +135,7 @@ GEMR_HD double qdk(double a, double b, double y) {
   const double q1 = __fma_rn(r, y, q0);
   if (((unsigned)__double2hiint(a) & 0x7fffffffu) - (523u << 20) < (1000u << 20)) return q1;
   if (a == 0.0) return q0;
-  return a / b;
+  return div_slow(a, b);
 #else
   (void)y;
   return a / b;
@@ -140,7 +154,7 @@ GEMR_HD double qdk_v(double a, double b, double y) {
   const bool yok = hy - (623u << 20) < (800u << 20);
   if ((ha - (523u << 20) < (1000u << 20)) & yok) return q1;
   if (a == 0.0 && yok) return q0;
-  return a / b;
+  return div_slow(a, b);
 #else
   (void)y;
   return a / b;
@@ -155,6 +169,38 @@ GEMR_HD double rcp_dev(double b) {
   return 0.0;
 #endif
 }
+
+// How the rate bodies divide by a constant (c) and by a run-time value with its reciprocal (v).
+// ExactQ tests every numerator.  FastQ (device) tests none: the caller has shown for all of
+// a body's inputs that no numerator, quotient or remainder leaves the normal range; the
+// remainder is formed negated, so a zero numerator's quotient keeps its sign.  Both give the
+// IEEE quotient.
+struct ExactQ {
+  static constexpr bool fast = false;
+  static GEMR_HD double c(double a, double b, double y) { return qdk(a, b, y); }
+  static GEMR_HD double v(double a, double b, double y) { return qdk_v(a, b, y); }
+};
+#ifdef __CUDACC__
+struct FastQ {
+  static constexpr bool fast = true;
+  static __device__ __forceinline__ double c(double a, double b, double y) {
+    const double q0 = a * y;
+    return __fma_rn(-__fma_rn(q0, b, -a), y, q0);
+  }
+  static __device__ __forceinline__ double v(double a, double b, double y) { return c(a, b, y); }
+};
+#endif
+
+// The state of one cell, species by species: element access to the ghosted blocks
+struct CellFields {
+  const double *ns, *vs1, *vs2, *vs3, *Ts;
+  long long k, ng;
+  GEMR_HD double n(int j) const { return ns[j * ng + k]; }
+  GEMR_HD double u1(int j) const { return vs1[j * ng + k]; }
+  GEMR_HD double u2(int j) const { return vs2[j * ng + k]; }
+  GEMR_HD double u3(int j) const { return vs3[j * ng + k]; }
+  GEMR_HD double T(int j) const { return Ts[j * ng + k]; }
+};
 
 // x**0.5 and x**1.5 of the collision and reaction fits.  The host build calls pow, as the
 // reference does; the device forms them from its correctly rounded square root (x**0.5
@@ -206,14 +252,22 @@ struct CoulPair {
   double P, Phi, Psi;  // Teff**1.5, Phi, Psi
   double yP;           // RN(1/P) on the device (rcp_dev)
 };
+template <class Q = ExactQ>
 GEMR_HD CoulPair coulomb_pair(const View& v, int isp, int isp2, double ts1, double ts2, double v1, double v2) {
   const double ms1 = v.ms[isp], ms2 = v.ms[isp2];
-  const double Teff = (ms2 * ts1 + ms1 * ts2) / (ms2 + ms1);
   CoulPair q;
+  double Teff, W;
+  if (Q::fast) {  // the same quotients from the host's tables
+    const double mred = v.mred[isp][isp2];
+    Teff = Q::c(ms2 * ts1 + ms1 * ts2, ms2 + ms1, v.yms[isp][isp2]);
+    W = fabs(v1 - v2) / sqrt(Q::c(2 * KB_ * Teff, mred, v.ymred[isp][isp2]));
+  } else {
+    Teff = (ms2 * ts1 + ms1 * ts2) / (ms2 + ms1);
+    const double mred = ms1 * ms2 / (ms1 + ms2);
+    W = fabs(v1 - v2) / sqrt(2 * KB_ * Teff / mred);
+  }
   q.P = pow_3half(Teff);
   q.yP = rcp_dev(q.P);
-  const double mred = ms1 * ms2 / (ms1 + ms2);
-  const double W = fabs(v1 - v2) / sqrt(2 * KB_ * Teff / mred);
   q.Psi = exp(-(W * W));
   if (W < 0.1)
     q.Phi = 1;
@@ -231,7 +285,7 @@ struct DirectPairs {
 
 // collisions.f90:117-159 for one cell: nu, Phi, Psi of species isp with isp2 (zero if equal);
 // the pair's symmetric part comes from `pairs`
-template <class Pairs>
+template <class Q, class Pairs>
 GEMR_HD void coulomb_colln(const View& v, int isp, int isp2, double ns2, double ts1, double ts2, double v1, double v2,
                            double& nu, double& Phi, double& Psi, const Pairs& pairs) {
   if (isp == isp2) {
@@ -239,7 +293,7 @@ GEMR_HD void coulomb_colln(const View& v, int isp, int isp2, double ns2, double 
     return;
   }
   const CoulPair q = pairs(v, isp, isp2, ts1, ts2, v1, v2);
-  nu = qdk_v(Coll::csj(isp, isp2) * ns2 * 1e-6, q.P, q.yP);
+  nu = Q::v(Coll::csj(isp, isp2) * ns2 * 1e-6, q.P, q.yP);
   Phi = q.Phi;
   Psi = q.Psi;
 }
@@ -387,39 +441,43 @@ GEMR_HD void continuity_cell(const View& v, long long c, const double* nn, const
 
 // ---- energy: index t = isp * ncell + c ----------------------------------------------------
 // nn: interior (lx1,lx2,lx3, O N2 O2 H ...); the rest as continuity_cell
-template <class Pairs = DirectPairs>
-GEMR_HD void energy_rate(const View& v, long long t, const double* nn, const double* vn1, const double* vn2,
-                         const double* vn3, const double* Tn, const double* ns, const double* vs1, const double* vs2,
-                         const double* vs3, const double* Ts, double* Pr, double* Lo, const Pairs& pairs = Pairs()) {
-  const long long nc = ncell(v);
-  const int isp = (int)(t / nc);
-  const long long c = t - isp * nc;
-  int i1, i2, i3;
-  cell_of(v, c, i1, i2, i3);
-  const long long k = gix(v, i1, i2, i3);
+// the body for species isp at interior cell c
+template <class Q, class Fld, class Pairs>
+GEMR_HD void energy_at(const View& v, int isp, long long c, const double* nn, const double* vn1, const double* vn2,
+                       const double* vn3, const double* Tn, const Fld& F, double* Pr, double* Lo, const Pairs& pairs) {
+  const long long nc = ncell(v), t = isp * nc + c;
   const double tn = Tn[c];
   const double ms = v.ms[isp], gm1 = v.gam[isp] - 1;
-  const double nsk = ns[isp * v.ng + k], tsk = Ts[isp * v.ng + k];
-  const double u1 = vs1[isp * v.ng + k], u2 = vs2[isp * v.ng + k], u3 = vs3[isp * v.ng + k];
+  const double nsk = F.n(isp), tsk = F.T(isp);
+  const double u1 = F.u1(isp), u2 = F.u2(isp), u3 = F.u3(isp);
   double pr = 0.0, lo = 0.0;
-  for (int j = 0; j < NNEU; ++j) {  // with the neutrals
-    const double nu = maxwell_colln(isp, j, nn[j * nc + c], tn, tsk);
-    double fact = qdk(2 * nu, ms + Coll::mn(j), v.ymn[isp][j]);
-    pr = pr + nsk * ms * KB_ / gm1 * fact * tn;
-    lo = lo + ms * fact;
-    fact = qdk(fact * Coll::mn(j), 3, Y3);
+  {  // with the neutrals
     const double d1 = u1 - vn1[c], d2 = u2 - vn2[c], d3 = u3 - vn3[c];
-    pr = pr + nsk * ms / gm1 * ((d1 * d1) + (d2 * d2) + (d3 * d3)) * fact;
+    const double dd = (d1 * d1) + (d2 * d2) + (d3 * d3);
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+    for (int j = 0; j < NNEU; ++j) {
+      const double nu = maxwell_colln(isp, j, nn[j * nc + c], tn, tsk);
+      double fact = Q::c(2 * nu, ms + Coll::mn(j), v.ymn[isp][j]);
+      pr = pr + nsk * ms * KB_ / gm1 * fact * tn;
+      lo = lo + ms * fact;
+      fact = Q::c(fact * Coll::mn(j), 3, Y3);
+      pr = pr + nsk * ms / gm1 * dd * fact;
+    }
   }
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
   for (int j = 0; j < NSP; ++j) {  // with the charged species
-    const long long kj = j * v.ng + k;
     double nu, Phi, Psi;
-    coulomb_colln(v, isp, j, ns[kj], tsk, Ts[kj], u1, vs1[kj], nu, Phi, Psi, pairs);
-    double fact = qdk(2 * nu * Psi, ms + v.ms[j], v.yms[isp][j]);
-    pr = pr + nsk * ms * KB_ / gm1 * fact * Ts[kj];
+    const double tj = F.T(j), v1 = F.u1(j);
+    coulomb_colln<Q>(v, isp, j, F.n(j), tsk, tj, u1, v1, nu, Phi, Psi, pairs);
+    double fact = Q::c(2 * nu * Psi, ms + v.ms[j], v.yms[isp][j]);
+    pr = pr + nsk * ms * KB_ / gm1 * fact * tj;
     lo = lo + ms * fact;
-    fact = qdk(qdk(2 * nu * Phi, ms + v.ms[j], v.yms[isp][j]) * v.ms[j], 3, Y3);
-    const double d1 = u1 - vs1[kj], d2 = u2 - vs2[kj], d3 = u3 - vs3[kj];
+    fact = Q::c(Q::c(2 * nu * Phi, ms + v.ms[j], v.yms[isp][j]) * v.ms[j], 3, Y3);
+    const double d1 = u1 - v1, d2 = u2 - F.u2(j), d3 = u3 - F.u3(j);
     pr = pr + nsk * ms / gm1 * ((d1 * d1) + (d2 * d2) + (d3 * d3)) * fact;
   }
   if (isp == NSP - 1) {  // inelastic electron losses: rotational, then vibrational excitation
@@ -445,6 +503,19 @@ GEMR_HD void energy_rate(const View& v, long long t, const double* nn, const dou
   }
   Pr[t] = pr;
   Lo[t] = lo;
+}
+
+template <class Pairs = DirectPairs>
+GEMR_HD void energy_rate(const View& v, long long t, const double* nn, const double* vn1, const double* vn2,
+                         const double* vn3, const double* Tn, const double* ns, const double* vs1, const double* vs2,
+                         const double* vs3, const double* Ts, double* Pr, double* Lo, const Pairs& pairs = Pairs()) {
+  const long long nc = ncell(v);
+  const int isp = (int)(t / nc);
+  const long long c = t - isp * nc;
+  int i1, i2, i3;
+  cell_of(v, c, i1, i2, i3);
+  energy_at<ExactQ>(v, isp, c, nn, vn1, vn2, vn3, Tn, CellFields{ns, vs1, vs2, vs3, Ts, gix(v, i1, i2, i3), v.ng}, Pr,
+                    Lo, pairs);
 }
 
 // ---- momentum: index t = isp * ncell + c --------------------------------------------------
@@ -498,17 +569,15 @@ struct DirectX1 {
 
 // nn: interior (lx1,lx2,lx3, O N2 O2 H ...); vn1, Tn, alt, g1: interior; Q: interior
 // (lx1,lx2,lx3,lsp); ns, vs1..3, Ts, E1: ghosted
-template <class Pairs = DirectPairs, class X1 = DirectX1>
-GEMR_HD void momentum_rate(const View& v, long long t, const double* nn, const double* vn1, const double* Tn,
-                           const double* ns, const double* vs1, const double* vs2, const double* vs3, const double* Ts,
-                           const double* E1, const double* Q, const double* alt, const double* g1, double* Pr,
-                           double* Lo, const Pairs& pairs = Pairs(), const X1& x1 = X1()) {
-  const long long nc = ncell(v);
-  const int isp = (int)(t / nc);
-  const long long c = t - isp * nc;
-  int i1, i2, i3;
-  cell_of(v, c, i1, i2, i3);
-  const long long kg = gix(v, i1, i2, i3), k = kg + isp * v.ng;
+// the body for species isp at interior cell c = (i1, i2, i3)
+template <class Qt, class Fld, class Pairs, class X1>
+GEMR_HD void momentum_at(const View& v, int isp, long long c, int i1, int i2, int i3, const double* nn,
+                         const double* vn1, const double* Tn, const double* ns, const double* Ts, const Fld& F,
+                         const double* E1, const double* Q, const double* alt, const double* g1, double* Pr, double* Lo,
+                         const Pairs& pairs, const X1& x1) {
+  const long long nc = ncell(v), t = isp * nc + c;
+  const long long kg = gix(v, i1, i2, i3);
+  const double nsk = F.n(isp), tsk = F.T(isp), u1 = F.u1(isp), u2 = F.u2(isp), u3 = F.u3(isp);
   const double ms = v.ms[isp];
   const X1Div q = x1_div(v, i1, i2, i3);
   const double h1 = q.h1, h2 = hm(v.h2, v, i1, i2, i3), h3 = hm(v.h3, v, i1, i2, i3);
@@ -524,31 +593,51 @@ GEMR_HD void momentum_rate(const View& v, long long t, const double* nn, const d
   const double epol = x1.epol(v, ns, Ts, i1, kg, km, kp, q);
   // pressure * d log(pressure)/dx1 and dQ/dx1
   const long long s0 = (long long)isp * v.ng;
-  const double pres = ns[s0 + kg] * KB_ * Ts[s0 + kg];
+  const double pres = nsk * KB_ * tsk;
   const double pg = x1.pg(v, ns, Ts, s0, i1, kg, km, kp, q);
   const long long qb = (long long)isp * nc;
   const long long cm = c - (i1 - im), cp = c + (ip - i1);
   const double gq = dx1_line(v, i1, Q[qb + cm], Q[qb + c], Q[qb + cp], q);
   double pr = 0.0, lo = 0.0;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
   for (int j = 0; j < NNEU; ++j) {  // with the neutrals
-    const double nu = maxwell_colln(isp, j, nn[j * nc + c], Tn[c], Ts[k]);
+    const double nu = maxwell_colln(isp, j, nn[j * nc + c], Tn[c], tsk);
     lo = lo + nu;
-    pr = pr + ns[k] * ms * nu * vn1[c];
+    pr = pr + nsk * ms * nu * vn1[c];
   }
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
   for (int j = 0; j < NSP; ++j) {  // with the charged species
     double nu, Phi, Psi;
-    const long long k2 = kg + (long long)j * v.ng;
-    coulomb_colln(v, isp, j, ns[k2], Ts[k], Ts[k2], vs1[k], vs1[k2], nu, Phi, Psi, pairs);
+    const double v1 = F.u1(j);
+    coulomb_colln<Qt>(v, isp, j, F.n(j), tsk, F.T(j), u1, v1, nu, Phi, Psi, pairs);
     lo = lo + nu * Phi;
-    pr = pr + ns[k] * ms * nu * Phi * vs1[k2];
+    pr = pr + nsk * ms * nu * Phi * v1;
   }
   const double ionpress = pres * pg;
   const double h1h2h3 = h1 * h2 * h3;
-  const double geom = (vs2[k] * vs2[k] * h3 * dh2 + vs3[k] * vs3[k] * h2 * dh3) * ns[k] * ms / h1h2h3;
+  const double geom = (u2 * u2 * h3 * dh2 + u3 * u3 * h2 * dh3) * nsk * ms / h1h2h3;
   const double e1f = (alt[c] < 100e3) ? 0.0 : E1[kg];
-  pr = pr + ns[k] * v.qs[isp] * (e1f + epol) - ionpress - gq + geom + ns[k] * ms * g1[c];
+  pr = pr + nsk * v.qs[isp] * (e1f + epol) - ionpress - gq + geom + nsk * ms * g1[c];
   Pr[t] = pr;
   Lo[t] = lo;
+}
+
+template <class Pairs = DirectPairs, class X1 = DirectX1>
+GEMR_HD void momentum_rate(const View& v, long long t, const double* nn, const double* vn1, const double* Tn,
+                           const double* ns, const double* vs1, const double* vs2, const double* vs3, const double* Ts,
+                           const double* E1, const double* Q, const double* alt, const double* g1, double* Pr,
+                           double* Lo, const Pairs& pairs = Pairs(), const X1& x1 = X1()) {
+  const long long nc = ncell(v);
+  const int isp = (int)(t / nc);
+  const long long c = t - isp * nc;
+  int i1, i2, i3;
+  cell_of(v, c, i1, i2, i3);
+  momentum_at<ExactQ>(v, isp, c, i1, i2, i3, nn, vn1, Tn, ns, Ts,
+                      CellFields{ns, vs1, vs2, vs3, Ts, gix(v, i1, i2, i3), v.ng}, E1, Q, alt, g1, Pr, Lo, pairs, x1);
 }
 
 }  // namespace gemr

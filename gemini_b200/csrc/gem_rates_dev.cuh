@@ -50,42 +50,113 @@ struct SmemPairs {
   }
 };
 
-// this thread's three pairs of cell c (ghosted index k), into the table
-__device__ __forceinline__ void fill_pairs(const gemr::View& v, int isp, int lane, long long k,
-                                           const double* __restrict__ vs1, const double* __restrict__ Ts,
-                                           PairTab& tab) {
-  const double t1 = Ts[isp * v.ng + k], u1 = vs1[isp * v.ng + k];
-#pragma unroll
+// The block's 32 cells in shared memory: n, v1, v2, v3, T of each species, loaded by the warp
+// of that species and read by all of them.
+struct CellTab {
+  double f[5][LSP][kRateCells];
+};
+struct SmemFields {
+  const CellTab* tab;
+  int lane;
+  __device__ __forceinline__ double n(int j) const { return tab->f[0][j][lane]; }
+  __device__ __forceinline__ double u1(int j) const { return tab->f[1][j][lane]; }
+  __device__ __forceinline__ double u2(int j) const { return tab->f[2][j][lane]; }
+  __device__ __forceinline__ double u3(int j) const { return tab->f[3][j][lane]; }
+  __device__ __forceinline__ double T(int j) const { return tab->f[4][j][lane]; }
+};
+
+// |x| in [2^lo, 2^hi), read from the exponent
+__device__ __forceinline__ bool exp_in(double x, int lo, int hi) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((unsigned)(1023 + lo) << 20) < ((unsigned)(hi - lo) << 20);
+}
+
+// FastQ's condition for the exchange rates, with margin: densities in [2^-350, 2^200) (the
+// floor is 1e-100), temperatures in [2^-20, 2^100), neutral densities 0 or in [2^-300, 2^200),
+// and of each pair Psi in [2^-250, 1] and Phi 0 or in [2^-100, 2^100).  Then P is in
+// [2^-30, 2^150), nu at least 2^-550, the numerators at least 2^-900 and their quotients by
+// masses (2^-101 .. 2^-82) and by 3 above 2^-960: nothing leaves the normal range.  Each warp
+// tests its species, its pairs and (warps 0..3) one neutral; the block takes the fast body
+// only if all pass.
+__device__ __forceinline__ bool state_ok(double n, double T) { return exp_in(n, -350, 200) && exp_in(T, -20, 100); }
+__device__ __forceinline__ bool pair_ok(const gemr::CoulPair& q) {
+  return exp_in(q.Psi, -250, 1) && (exp_in(q.Phi, -100, 100) || q.Phi == 0.0);
+}
+
+// this thread's three pairs of its cell, into the table; returns whether the fast bodies may
+// use them
+template <class Q>
+__device__ __forceinline__ bool fill_pairs(const gemr::View& v, int isp, int lane, const SmemFields& F, PairTab& tab) {
+  const double t1 = F.T(isp), u1 = F.u1(isp);
+  bool ok = true;
+#pragma unroll 1
   for (int d = 1; d <= 3; ++d) {
     const int j = (isp + d < LSP) ? isp + d : isp + d - LSP;
-    const gemr::CoulPair q = gemr::coulomb_pair(v, isp, j, t1, Ts[j * v.ng + k], u1, vs1[j * v.ng + k]);
+    const gemr::CoulPair q = gemr::coulomb_pair<Q>(v, isp, j, t1, F.T(j), u1, F.u1(j));
     const int p = isp * 3 + d - 1;
     tab.P[p][lane] = q.P;
     tab.Phi[p][lane] = q.Phi;
     tab.Psi[p][lane] = q.Psi;
     tab.yP[p][lane] = q.yP;
+    ok = ok && pair_ok(q);
   }
+  return ok;
 }
 
-// Five 7-warp blocks per SM (56 registers, 112 bytes spilled): 11.2 -> 10.3 ms on the
-// 384x192x192 dipole grid against its natural 72 registers and four blocks.
+// Loads the block's cells (the warp of species isp its own), then fills the pair table; true
+// when the fast bodies apply to the whole block.  The pairs' own quotients by masses need
+// only the temperatures' range.
+__device__ __forceinline__ bool load_cells(const gemr::View& v, const double* __restrict__ nn, int isp, int lane, bool in,
+                                           long long c, long long k, const double* __restrict__ fv, CellTab& cells,
+                                           PairTab& tab) {
+  bool ok = true;
+  if (in) {
+    double x[5];
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
+      x[f] = fv[(long long)(f * LSP + isp) * v.ng + k];
+      cells.f[f][isp][lane] = x[f];
+    }
+    ok = state_ok(x[0], x[4]);
+    if (isp < gemr::NNEU) {
+      const double q = nn[isp * gemr::ncell(v) + c];
+      ok = ok && (exp_in(q, -300, 200) || q == 0.0);
+    }
+  }
+  ok = __syncthreads_and(ok);
+  const SmemFields F{&cells, lane};
+  bool pok = true;
+  if (in) {
+    if (ok) pok = fill_pairs<gemr::FastQ>(v, isp, lane, F, tab);
+    else pok = fill_pairs<gemr::ExactQ>(v, isp, lane, F, tab);
+  }
+  return __syncthreads_and(pok) && ok;
+}
+
+// Bound by instruction issue (65%, FP64 pipe 38%).  Five 7-warp blocks per SM (56 registers,
+// 76 bytes spilled): 1.91 ms for 384x96x96, four blocks 2.03, six 2.17; the loops over partners
+// are not unrolled (2.02 ms unrolled: the code outgrows the instruction cache).  Before the
+// fast quotients and the shared cell table, 2.83 ms.
 __global__ void __launch_bounds__(kRateThreads, 5) kr_energy(gemr::View v, RateIn in, const double* __restrict__ fv,
                                                           double* __restrict__ Pr, double* __restrict__ Lo) {
   __shared__ PairTab tab;
+  __shared__ CellTab cells;
   const int isp = threadIdx.x / kRateCells, lane = threadIdx.x % kRateCells;
   const long long nc = gemr::ncell(v);
   const long long c = (long long)blockIdx.x * kRateCells + lane;
-  const double *ns = fv, *vs1 = fv + LSP * v.ng, *vs2 = fv + 2 * LSP * v.ng, *vs3 = fv + 3 * LSP * v.ng,
-               *Ts = fv + 4 * LSP * v.ng;
+  long long k = 0;
   if (c < nc) {
     int i1, i2, i3;
     gemr::cell_of(v, c, i1, i2, i3);
-    fill_pairs(v, isp, lane, gemr::gix(v, i1, i2, i3), vs1, Ts, tab);
+    k = gemr::gix(v, i1, i2, i3);
   }
-  __syncthreads();
-  if (c < nc)
-    gemr::energy_rate(v, isp * nc + c, in.nn, in.vn1, in.vn2, in.vn3, in.Tn, ns, vs1, vs2, vs3, Ts, Pr, Lo,
-                      SmemPairs{&tab, lane});
+  const bool fast = load_cells(v, in.nn, isp, lane, c < nc, c, k, fv, cells, tab);
+  if (c >= nc) return;
+  const SmemFields F{&cells, lane};
+  const SmemPairs pairs{&tab, lane};
+  if (fast)
+    gemr::energy_at<gemr::FastQ>(v, isp, c, in.nn, in.vn1, in.vn2, in.vn3, in.Tn, F, Pr, Lo, pairs);
+  else
+    gemr::energy_at<gemr::ExactQ>(v, isp, c, in.nn, in.vn1, in.vn2, in.vn3, in.Tn, F, Pr, Lo, pairs);
 }
 
 // x1 log-gradient terms from values the block formed once: the electrons' ambipolar term
@@ -107,10 +178,10 @@ struct SharedX1 {
 // are the adjacent lanes (c +- 1), except across the block's edges (lanes 0 and 31), which
 // form that one neighbour's log themselves.  At the line ends the missing side is the cell
 // itself, as the direct form's clamped neighbour index gives.
-// Five 7-warp blocks per SM (56 registers, 132 bytes spilled): each SM sub-partition holds a
-// quarter of the register file, so at its natural 93 registers (96 allocated) only 5 warps
-// fit per sub-partition and two blocks per SM (16.2 ms on the 384x192x192 dipole grid;
-// 72 registers, four blocks: 10.1 ms; 56: 9.95 ms).
+// Five 7-warp blocks per SM (56 registers): each SM sub-partition holds a quarter of the
+// register file, so at the kernel's natural 90-odd registers only 5 warps fit per
+// sub-partition and two blocks per SM.  384x96x96: 2.08 ms, four blocks 2.28, six 2.26; before
+// the fast quotients and the shared cell table, 2.78 ms.
 __global__ void __launch_bounds__(kRateThreads, 5) kr_momentum(gemr::View v, RateIn in, const double* __restrict__ fv,
                                                             const double* __restrict__ E1,
                                                             const double* __restrict__ Q,
@@ -118,23 +189,23 @@ __global__ void __launch_bounds__(kRateThreads, 5) kr_momentum(gemr::View v, Rat
                                                             const double* __restrict__ g1, double* __restrict__ Pr,
                                                             double* __restrict__ Lo) {
   __shared__ PairTab tab;
+  __shared__ CellTab cells;
   __shared__ double s_epol[kRateCells];
   const int isp = threadIdx.x / kRateCells, lane = threadIdx.x % kRateCells;
   const long long nc = gemr::ncell(v);
   const long long c = (long long)blockIdx.x * kRateCells + lane;
   const bool ok = c < nc;
-  const double *ns = fv, *vs1 = fv + LSP * v.ng, *vs2 = fv + 2 * LSP * v.ng, *vs3 = fv + 3 * LSP * v.ng,
-               *Ts = fv + 4 * LSP * v.ng;
+  const double *ns = fv, *Ts = fv + 4 * LSP * v.ng;
   const long long s0 = (long long)isp * v.ng;
   int i1 = 1, i2 = 1, i3 = 1;
   long long kg = 0;
-  double l0 = 0.0;
   if (ok) {
     gemr::cell_of(v, c, i1, i2, i3);
     kg = gemr::gix(v, i1, i2, i3);
-    fill_pairs(v, isp, lane, kg, vs1, Ts, tab);
-    l0 = log(ns[s0 + kg] * gemr::KB_ * Ts[s0 + kg]);
   }
+  const bool fast = load_cells(v, in.nn, isp, lane, ok, c, kg, fv, cells, tab);
+  const SmemFields F{&cells, lane};
+  const double l0 = ok ? log(F.n(isp) * gemr::KB_ * F.T(isp)) : 0.0;
   double lm = __shfl_up_sync(0xffffffffu, l0, 1), lp = __shfl_down_sync(0xffffffffu, l0, 1);
   if (ok) {
     if (i1 == 1) lm = l0;
@@ -149,13 +220,19 @@ __global__ void __launch_bounds__(kRateThreads, 5) kr_momentum(gemr::View v, Rat
         lp = x;
     }
     if (isp == LSP - 1)
-      s_epol[lane] = gemr::KB_ * Ts[s0 + kg] / v.qs[LSP - 1] *
+      s_epol[lane] = gemr::KB_ * F.T(isp) / v.qs[LSP - 1] *
                      gemr::dx1_line(v, i1, lm, l0, lp, gemr::x1_div(v, i1, i2, i3));
   }
   __syncthreads();
-  if (ok)
-    gemr::momentum_rate(v, isp * nc + c, in.nn, in.vn1, in.Tn, ns, vs1, vs2, vs3, Ts, E1, Q, alt, g1, Pr, Lo,
-                        SmemPairs{&tab, lane}, SharedX1{s_epol[lane], lm, l0, lp});
+  if (!ok) return;
+  const SmemPairs pairs{&tab, lane};
+  const SharedX1 x1{s_epol[lane], lm, l0, lp};
+  if (fast)
+    gemr::momentum_at<gemr::FastQ>(v, isp, c, i1, i2, i3, in.nn, in.vn1, in.Tn, ns, Ts, F, E1, Q, alt, g1, Pr, Lo, pairs,
+                                   x1);
+  else
+    gemr::momentum_at<gemr::ExactQ>(v, isp, c, i1, i2, i3, in.nn, in.vn1, in.Tn, ns, Ts, F, E1, Q, alt, g1, Pr, Lo, pairs,
+                                    x1);
 }
 
 gemr::View rate_view(const gem_grid* g) {
@@ -186,7 +263,11 @@ gemr::View rate_view(const gem_grid* g) {
   const double mn[gemr::NNEU] = {16 * gemr::AMU_, 28 * gemr::AMU_, 32 * gemr::AMU_, 1 * gemr::AMU_};  // Coll::mn
   for (int i = 0; i < LSP; ++i) {
     for (int j = 0; j < gemr::NNEU; ++j) v.ymn[i][j] = 1.0 / (v.ms[i] + mn[j]);
-    for (int j = 0; j < LSP; ++j) v.yms[i][j] = 1.0 / (v.ms[i] + v.ms[j]);
+    for (int j = 0; j < LSP; ++j) {
+      v.yms[i][j] = 1.0 / (v.ms[i] + v.ms[j]);
+      v.mred[i][j] = v.ms[i] * v.ms[j] / (v.ms[i] + v.ms[j]);  // as coulomb_pair forms it
+      v.ymred[i][j] = 1.0 / v.mred[i][j];
+    }
   }
   return v;
 }

@@ -45,9 +45,17 @@ GEMS_HD long long ncell(const View& v) { return (long long)v.lx1 * v.lx2 * v.lx3
 // ghosted linear index k -> whether it is an interior cell, and then its column-major
 // interior index c
 GEMS_HD bool interior(const View& v, long long k, long long& c) {
-  const int i1 = (int)(k % v.s2) - 1;
-  const int i2 = (int)((k / v.s2) % (v.lx2 + 4)) - 1;
-  const int i3 = (int)(k / v.s3) - 1;
+  int i1, i2, i3;
+  if ((unsigned long long)k <= 0xffffffffull) {  // 32-bit quotients where the index fits
+    const unsigned u = (unsigned)k, r = u / (unsigned)v.s2, q = r / (unsigned)(v.lx2 + 4);
+    i1 = (int)(u - r * (unsigned)v.s2) - 1;
+    i2 = (int)(r - q * (unsigned)(v.lx2 + 4)) - 1;
+    i3 = (int)q - 1;
+  } else {
+    i1 = (int)(k % v.s2) - 1;
+    i2 = (int)((k / v.s2) % (v.lx2 + 4)) - 1;
+    i3 = (int)(k / v.s3) - 1;
+  }
   if (i1 < 1 || i1 > v.lx1 || i2 < 1 || i2 > v.lx2 || i3 < 1 || i3 > v.lx3) return false;
   c = (long long)(i1 - 1) + (long long)v.lx1 * ((i2 - 1) + (long long)v.lx2 * (i3 - 1));
   return true;
