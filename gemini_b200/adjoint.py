@@ -47,7 +47,7 @@ class DiffProblem:
         self._sa = None  # gem_step_adjoint workspaces (the backward's replay slots), made on first use
         self._side = None  # the replay stream of the pipelined backward
         self.replay_slots = True  # recompute by replay + finish when k+1 workspaces fit
-        self._dtt = {}
+        self._dtt = None
         self._capturing = False
         self._graphs = {}  # (Ttop given) -> captured step VJP
         self.vjp_graph = True
@@ -83,7 +83,7 @@ class DiffProblem:
     # -- CUDA state plumbing -------------------------------------------------------------
     def _load(self, ns, vs1, Ts, lo, hi, Ttop):
         fv = self.ds.fluidvars.view(self.shape)
-        fv.copy_(self.base)
+        fv[2 * LSP:4 * LSP] = self.base[2 * LSP:4 * LSP]
         fv[0:LSP] = ns
         fv[LSP:2 * LSP] = vs1
         fv[4 * LSP:] = Ts
@@ -101,20 +101,16 @@ class DiffProblem:
                 self.v1i[..., 0].clone(), self.v1i[..., -1].clone())
 
     def dt_tensor(self, j: int):
-        """The step's dt as a cached 1-element device tensor."""
+        """The step's dt as a cached 1-element device tensor.  The schedule is copied once, by
+        a copy the host waits for, so that any stream may read it afterwards."""
         import torch
 
-        t = self._dtt.get(j)
-        if t is None:
-            t = torch.full((1,), self.dts[j], dtype=torch.float64, device=self.base.device)
-            self._dtt[j] = t
-        return t
+        if self._dtt is None:
+            self._dtt = torch.tensor(self.dts, dtype=torch.float64, device=self.base.device)
+        return self._dtt[j:j + 1]
 
     def cuda_step(self, j: int) -> None:
-        import torch
-
-        dt = torch.full((1,), self.dts[j], dtype=torch.float64, device=self.ds.fluidvars.device)
-        F.fluid_adv(self.cfg, self.ds, dt)
+        F.fluid_adv(self.cfg, self.ds, self.dt_tensor(j))
 
     def initial_state(self, n0, Ttop=None):
         """Full-layout initial state with the ion densities n0 (6, lx3, lx2, lx1) in the
@@ -500,6 +496,14 @@ def _backward_cuda(P: "DiffProblem", ckpt, starts, Ttop, cot, g_top):
     n = P.nsteps
     kmax = max((starts[i + 1] if i + 1 < len(starts) else n) - starts[i] for i in range(len(starts)))
     have = sum(1 for h in (P._sa or []) if h is not None)
+    if P.replay_slots and have > kmax:
+        # the workspaces exist: asking the driver for its free memory (0.6 ms) is left out until
+        # torch itself runs short; the backward then starts again below
+        try:
+            return _backward_cuda_slots(P, ckpt, starts, Ttop, cot, g_top, kmax + 1)
+        except torch.cuda.OutOfMemoryError:
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
     F1 = 8 * LSP * (P.grid.lx1 + 4) * (P.grid.lx2 + 4) * (P.grid.lx3 + 4)
     need = max(0, kmax + 1 - have) * P.workspace_bytes() + 2 * kmax * 3 * F1
     # the recompute's diffusion scratch first; the workspaces are raw cudaMalloc, which cannot

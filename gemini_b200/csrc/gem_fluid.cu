@@ -241,6 +241,23 @@ int launch_sweep(const gem_grid* g, int dim, bool fused, SweepArgs a, int nsp, c
   return launch_sweep_t<3, false>(g, a, nsp, st);
 }
 
+// a direction's three fields out of place (the differentiable path's replay)
+int launch_sweep_tri(const gem_grid* g, int dim, const SweepTri& T, cudaStream_t st) {
+  const Dims& d = g->dev.d;
+  const bool u = g->dev.unit != 0;
+  const dim3 block(32, LSP);
+  if (dim == 1) {
+    auto kern = u ? k_sweep_tri_x1<true> : k_sweep_tri_x1<false>;
+    kern<<<dim3(d.lx2, d.lx3, 3), block, 0, st>>>(T);
+  } else {
+    auto kern = dim == 3 ? (u ? k_sweep_tri<3, true> : k_sweep_tri<3, false>)
+                         : (u ? k_sweep_tri<2, true> : k_sweep_tri<2, false>);
+    kern<<<dim3((d.lx1 + 31) / 32, dim == 3 ? d.lx2 : d.lx3, 3 * sweep_parts(d, dim)), block, 0, st>>>(T);
+  }
+  GEM_LAUNCHED("k_sweep_tri");
+  return GEM_OK;
+}
+
 int launch_ghost_fill(const gem_grid* g, Blocks B, const double* vs1i, int lsp, bool fused,
                       cudaStream_t st) {
   const Dims& d = g->dev.d;

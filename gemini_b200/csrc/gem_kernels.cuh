@@ -730,6 +730,21 @@ struct SweepArgs {
   // fused sweeps out of place (all null: in place): the densities between x3 and x2, and the
   // momentum and energy densities between x1 and x2, in blocks of the state blocks' layout
   double *nsB = nullptr, *rvB = nullptr, *reB = nullptr;
+  double* out = nullptr;  // standalone sweep out of place: the swept field's block
+};
+
+// The standalone sweeps of one direction's three fields out of place, in one launch: n, rv
+// (frank 1 along x2, x3) of six species and re of seven.
+struct SweepTri {
+  SweepArgs a;
+  double *src0, *src1, *src2, *dst0, *dst1, *dst2;
+  __device__ __forceinline__ SweepArgs field(int f, int dim) const {
+    SweepArgs p = a;
+    p.B.F = p.B.A = f == 0 ? src0 : f == 1 ? src1 : src2;
+    p.out = f == 0 ? dst0 : f == 1 ? dst1 : dst2;
+    p.which = (f == 1 && dim != 1) ? 1 : 0;
+    return p;
+  }
 };
 
 // ---- the scheme of one field at one position -----------------------------------------------
@@ -875,9 +890,9 @@ __device__ __forceinline__ void cp_async_wait() {
 // come after the compression sub-step).
 // INV (x3 sweep, tabulated metrics that do not vary along x3): the line's metrics are read
 // once.
-// seg, nseg: this thread's part of the line; more than one part needs the fused sweeps'
-// separate inputs and outputs (SweepArgs::nsB ...), since a part's first cells are
-// neighbours of cells that another thread updates.
+// seg, nseg: this thread's part of the line; more than one part needs separate inputs and
+// outputs (SweepArgs::nsB ..., out), since a part's first cells are neighbours of cells that
+// another thread updates.
 template <int DIM, bool UNIT, bool FUSED, int PERM = 2, bool KEEPRE = false, bool INV = false>
 __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb, int seg = 0, int nseg = 1) {
   const GridDev& G = P.G;
@@ -938,9 +953,10 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb, i
     }
   } else {
     fr1 = P.which == 1;
-    dst[0] = ((P.which == 0) ? B.ns(s) : (P.which == 1) ? B.rv(s) : B.re(s)) + base;
+    src[0] = ((P.which == 0) ? B.ns(s) : (P.which == 1) ? B.rv(s) : B.re(s)) + base;
+    src[1] = src[2] = src[0];
+    dst[0] = (P.out ? P.out + (long long)s * d.ng : (P.which == 0) ? B.ns(s) : (P.which == 1) ? B.rv(s) : B.re(s)) + base;
     dst[1] = dst[2] = dst[0];
-    src[0] = src[1] = src[2] = dst[0];
     // face j in the work arrays (full 3-D layout), at [(j-1)*vst]
     vel = P.vsi + (long long)s * ((DIM == 3) ? nf3(d) : nf2(d)) + ((DIM == 3) ? f3i(d, aa, b, 1) : f2i(d, aa, 1, b));
   }
@@ -1001,6 +1017,7 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb, i
       dst[1][k] = conv_rv(src[0][k], src[1][k], s);
       dst[2][k] = conv_re(src[0][k], src[2][k], s);
     }
+    if (!FUSED && P.out && valid) dst[0][off(1)] = src[0][off(1)];
     return;
   }
 
@@ -1306,6 +1323,15 @@ __global__ void __launch_bounds__(224, GEM_MARCH_MINB) k_sweep_march(SweepArgs P
 }
 
 
+// three fields out of place (SweepTri); blockIdx.z: field + 3 * part of the line
+template <int DIM, bool UNIT>
+__global__ void __launch_bounds__(224, 2) k_sweep_tri(SweepTri T) {
+  const int f = blockIdx.z % 3;
+  if (threadIdx.y == LSP - 1 && f < 2) return;
+  b_sweep_march<DIM, UNIT, false>(T.field(f, DIM), VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x},
+                                  (int)blockIdx.z / 3, (int)gridDim.z / 3);
+}
+
 // ---- x1 sweep: lanes along the column ------------------------------------------------------
 // Lane l of chunk c handles position p = 32c + l - 1... the chunk covers p = 32c .. 32c+31 over
 // p = 0 .. lx1+1: the slope at cell p, the flux P(p) = ha2i(p)*phi(p) at face p, and the update
@@ -1341,7 +1367,8 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
   }
 #pragma unroll
   for (int f = 0; f < 3; ++f) src[f] = dst[f] = fld[f];
-  if constexpr (OOP) {
+  if constexpr (OOP && !FUSED) dst[0] = P.out + (long long)s * d.ng + col;
+  if constexpr (OOP && FUSED) {
     const long long so = (long long)s * d.ng + col;
     if (ion) src[0] = P.nsB + so;
     dst[0] = ion ? src[0] : P.reB + so;
@@ -1500,6 +1527,13 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
 template <bool UNIT, bool FUSED, bool OOP = false>
 __global__ void __launch_bounds__(224, OOP ? 2 : 3) k_sweep_x1(SweepArgs P) {
   b_sweep_x1<UNIT, FUSED, OOP>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
+}
+
+template <bool UNIT>
+__global__ void __launch_bounds__(224, 3) k_sweep_tri_x1(SweepTri T) {
+  const int f = blockIdx.z;
+  if (threadIdx.y == LSP - 1 && f < 2) return;
+  b_sweep_x1<UNIT, false, true>(T.field(f, 1), VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
 
