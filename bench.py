@@ -372,7 +372,7 @@ def run_b200(args, world, rank, local):
         cpu = {"value": v, "unit": UNIT, "cores": threads, "kind": "port", "sample": sample,
                "single_thread": single}
 
-    launches_per_step = 2 + 3 + 3 + 1 + (1 if g.lnull > 0 else 0) + 1
+    launches_per_step = 1 + 3 + 3 + 1 + (1 if g.lnull > 0 else 0) + 1
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True,

@@ -42,7 +42,7 @@ __global__ void kb_set_dt(const InstDev* inst, const double* dt_in, int ninst) {
   if (i < ninst) *inst[i].sw.dtp_w = dt_in[i];
 }
 
-// k_dt_finalize per instance
+// the time step of each instance from its maxima (k_dt_calc's formula)
 __global__ void kb_dt_finalize(const InstDev* inst, int ninst) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ninst) return;
@@ -83,12 +83,13 @@ __global__ void __launch_bounds__(128) kb_ghost_x3(const InstDev* __restrict__ i
   }
 }
 
-template <int DIM, bool UNIT, bool INV = false>
+// PERM 0: no instance is periodic (the x3 wrap values then take no registers)
+template <int DIM, bool UNIT, bool INV = false, int PERM = 2>
 __global__ void __launch_bounds__(224, 2) kb_sweep_march(const InstDev* __restrict__ inst, const Item* __restrict__ it, int n) {
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     const Item q = it[w];
     const InstDev& I = inst[q.x];
-    b_sweep_march<DIM, UNIT, true, 2, false, INV>(I.sw, VB{q.y, q.z, q.w});
+    b_sweep_march<DIM, UNIT, true, PERM, false, INV>(I.sw, VB{q.y, q.z, q.w});
     if (DIM == 2) __syncthreads();  // the epilogue's shared buffers are reused by the next item
   }
 }
@@ -152,11 +153,19 @@ enum BatchKernel { BK_DT = 0, BK_GX1, BK_GX2, BK_GX3, BK_SW3, BK_SW1, BK_SW2, BK
 struct BatchLaunch {
   int kernel = 0;
   int unit = 0;
-  bool inv = true;  // every instance's metrics are x3-invariant (x3 sweep)
+  bool inv = true;   // every instance's metrics are x3-invariant (x3 sweep)
+  bool open = true;  // no instance is periodic (x3 sweep)
   int grid = 0;
   std::vector<Item> items;
   Item* d_items = nullptr;
 };
+
+// the x3 sweep kernel of a launch's instances
+auto sweep3_kernel(const BatchLaunch& L) {
+  if (L.unit) return L.open ? kb_sweep_march<3, true, false, 0> : kb_sweep_march<3, true>;
+  if (L.inv) return L.open ? kb_sweep_march<3, false, true, 0> : kb_sweep_march<3, false, true>;
+  return L.open ? kb_sweep_march<3, false, false, 0> : kb_sweep_march<3, false>;
+}
 
 }  // namespace
 
@@ -211,9 +220,7 @@ int launch_grid(gem_batch* b, BatchLaunch& L) {
     case BK_GX1: return occupancy_grid(kb_ghost_x1, 128, 0, n, sc, &L.grid);
     case BK_GX2: return occupancy_grid(kb_ghost_x2, 128, 0, n, sc, &L.grid);
     case BK_GX3: return occupancy_grid(kb_ghost_x3, 128, 0, n, sc, &L.grid);
-    case BK_SW3: return u ? occupancy_grid(kb_sweep_march<3, true>, 32 * LSP, 0, n, sc, &L.grid)
-             : L.inv      ? occupancy_grid(kb_sweep_march<3, false, true>, 32 * LSP, 0, n, sc, &L.grid)
-                          : occupancy_grid(kb_sweep_march<3, false>, 32 * LSP, 0, n, sc, &L.grid);
+    case BK_SW3: return occupancy_grid(sweep3_kernel(L), 32 * LSP, 0, n, sc, &L.grid);
     case BK_SW1: return u ? occupancy_grid(kb_sweep_x1<true>, 32 * LSP, 0, n, sc, &L.grid)
                           : occupancy_grid(kb_sweep_x1<false>, 32 * LSP, 0, n, sc, &L.grid);
     case BK_SW2: return u ? occupancy_grid(kb_sweep_march<2, true>, 32 * LSP, 0, n, sc, &L.grid)
@@ -268,6 +275,7 @@ int batch_build_lists(gem_batch* b) {
           case BK_SW3: {
             BatchLaunch& L = launch_for(k, u);
             L.inv = L.inv && g->dev.c3 == 0;
+            L.open = L.open && !g->dev.flagper;
             add_items(L, i, gx13, d.lx2);
             break;
           }
@@ -333,9 +341,7 @@ int batch_enqueue(gem_batch* b, cudaStream_t st, bool fixed_dt = false) {
       case BK_GX2: kb_ghost_x2<<<L.grid, 128, 0, st>>>(I, L.d_items, n); break;
       case BK_GX3: kb_ghost_x3<<<L.grid, 128, 0, st>>>(I, L.d_items, n); break;
       case BK_SW3:
-        if (u) kb_sweep_march<3, true><<<L.grid, dim3(32, LSP), 0, st>>>(I, L.d_items, n);
-        else if (L.inv) kb_sweep_march<3, false, true><<<L.grid, dim3(32, LSP), 0, st>>>(I, L.d_items, n);
-        else kb_sweep_march<3, false><<<L.grid, dim3(32, LSP), 0, st>>>(I, L.d_items, n);
+        sweep3_kernel(L)<<<L.grid, dim3(32, LSP), 0, st>>>(I, L.d_items, n);
         break;
       case BK_SW1:
         if (u) kb_sweep_x1<true><<<L.grid, dim3(32, LSP), 0, st>>>(I, L.d_items, n);

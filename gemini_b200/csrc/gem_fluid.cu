@@ -80,6 +80,12 @@ unsigned grid_for(long long n, int threads, int per_sm = 8) {
   return (unsigned)b;
 }
 
+// blocks of the dt and CFL reductions: a block per x1 row up to the four an SM holds (eight, a
+// second partial wave: 96x32x32 20.4 us against 17.3; the same at 384x192x192)
+unsigned dt_blocks(const Dims& d) {
+  return (unsigned)std::min<long long>((long long)d.lx2 * d.lx3, (long long)num_sms() * 4);
+}
+
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 }  // namespace
@@ -118,6 +124,7 @@ struct gem_work {
   int has_src;
   double *Q, *Pr, *Lo;
   unsigned long long* acc;  // 32 slots: CFL maxima / counters
+  double* dtpart;           // dt_calc's maxima, 3*LSP per block of any grid (four per SM)
   long long nf1, nf2, nf3;
   // device staging of the host blocks for gem_fluid_adv_host, and its copy-out stream with
   // the events after the ghost fill, the ghost epilogue and the diffusion
@@ -741,6 +748,7 @@ int gem_work_create(const gem_grid* g, gem_work** out) {
   gem_work* w = new gem_work();
   w->vs1i = w->vs2i = w->vs3i = w->nn = w->Tn = w->dt = nullptr;
   w->acc = nullptr;
+  w->dtpart = nullptr;
   w->Ttop = nullptr;
   w->lu = nullptr;
   w->sweep = nullptr;
@@ -768,7 +776,8 @@ int gem_work_create(const gem_grid* g, gem_work** out) {
             {(void**)&w->nn, sizeof(double) * nc * 3},
             {(void**)&w->Tn, sizeof(double) * nc},
             {(void**)&w->dt, sizeof(double) * 4},
-            {(void**)&w->acc, sizeof(unsigned long long) * 32}};
+            {(void**)&w->acc, sizeof(unsigned long long) * 32},
+            {(void**)&w->dtpart, sizeof(double) * 3 * LSP * num_sms() * 4}};
   for (auto& a : al) {
     if (cudaMalloc(a.p, a.bytes) != cudaSuccess) {
       gem_work_destroy(w);
@@ -780,6 +789,11 @@ int gem_work_create(const gem_grid* g, gem_work** out) {
       return set_err(GEM_ECUDA, "cudaMemset failed");
     }
   }
+  // any stream may use the work object next (dt_calc counts its blocks from the zeroed acc)
+  if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    gem_work_destroy(w);
+    return set_err(GEM_ECUDA, "cudaStreamSynchronize failed");
+  }
   *out = w;
   return GEM_OK;
 }
@@ -790,7 +804,7 @@ int gem_work_destroy(gem_work* w) {
   for (cudaEvent_t e : w->ev)
     if (e) cudaEventDestroy(e);
   if (w->cs) cudaStreamDestroy(w->cs);
-  void* ps[] = {w->vs1i, w->vs2i, w->vs3i, w->nn, w->Tn, w->dt, w->acc, w->F, w->A, w->E, w->Ttop, w->lu, w->sweep, w->sub};
+  void* ps[] = {w->vs1i, w->vs2i, w->vs3i, w->nn, w->Tn, w->dt, w->acc, w->dtpart, w->F, w->A, w->E, w->Ttop, w->lu, w->sweep, w->sub};
   for (void* p : ps)
     if (p) cudaFree(p);
   delete w;
@@ -1065,16 +1079,11 @@ int gem_dt_calc_dev(const gem_grid* g, double tcfl, const double* fluidvars, gem
   if (check_grid(g) || !fluidvars || !w || !dt_out) return set_err(GEM_EINVAL, "null argument");
   cudaStream_t st = S(stream);
   w->timer.record(0, st);
-  GEM_CUDA(cudaMemsetAsync(w->acc, 0, 3 * LSP * sizeof(unsigned long long), st));
   Blocks B = blocks(g, const_cast<double*>(fluidvars), nullptr);
-  const unsigned nb = (unsigned)std::min<long long>((long long)g->dev.d.lx2 * g->dev.d.lx3, (long long)num_sms() * 8);
-  if (g->dev.unit)
-    k_dt_reduce<true, 0><<<nb, dim3(32, LSP), 0, st>>>(g->dev, B, w->acc, nullptr);
-  else
-    k_dt_reduce<false, 0><<<nb, dim3(32, LSP), 0, st>>>(g->dev, B, w->acc, nullptr);
-  GEM_LAUNCHED("k_dt_reduce");
-  k_dt_finalize<<<1, 32, 0, st>>>(w->acc, tcfl, dt_out);
-  GEM_LAUNCHED("k_dt_finalize");
+  const unsigned nb = dt_blocks(g->dev.d);
+  auto kern = g->dev.unit ? k_dt_calc<true> : k_dt_calc<false>;
+  kern<<<nb, dim3(32, LSP), 0, st>>>(g->dev, B, w->dtpart, w->acc + 30, tcfl, dt_out);
+  GEM_LAUNCHED("k_dt_calc");
   w->timer.record(1, st);
   return GEM_OK;
 }
@@ -1186,12 +1195,12 @@ int gem_maxcfl_dev(const gem_grid* g, const double* fluidvars, gem_work* w, cons
   cudaStream_t st = S(stream);
   GEM_CUDA(cudaMemsetAsync(w->acc + 24, 0, sizeof(unsigned long long), st));
   Blocks B = blocks(g, const_cast<double*>(fluidvars), nullptr);
-  const unsigned nb = (unsigned)std::min<long long>((long long)g->dev.d.lx2 * g->dev.d.lx3, (long long)num_sms() * 8);
+  const unsigned nb = dt_blocks(g->dev.d);
   if (g->dev.unit)
-    k_dt_reduce<true, 1><<<nb, dim3(32, LSP), 0, st>>>(g->dev, B, w->acc + 24, dt);
+    k_maxcfl<true><<<nb, dim3(32, LSP), 0, st>>>(g->dev, B, w->acc + 24, dt);
   else
-    k_dt_reduce<false, 1><<<nb, dim3(32, LSP), 0, st>>>(g->dev, B, w->acc + 24, dt);
-  GEM_LAUNCHED("k_dt_reduce");
+    k_maxcfl<false><<<nb, dim3(32, LSP), 0, st>>>(g->dev, B, w->acc + 24, dt);
+  GEM_LAUNCHED("k_maxcfl");
   k_maxcfl_finalize<<<1, 32, 0, st>>>(w->acc + 24, maxcfl_out);
   GEM_LAUNCHED("k_maxcfl_finalize");
   return GEM_OK;

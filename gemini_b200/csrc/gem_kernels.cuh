@@ -165,16 +165,15 @@ __device__ __forceinline__ double mdiv(double a, double b, double y) {
   return slow_div(a, b);
 }
 
-// mdiv without the fallback: clears ok when the quotient must be recomputed as a/b
+// mdiv without the fallback: clears ok when the quotient must be recomputed as a/b.  The
+// remainder is formed negated, so that a zero numerator's quotient keeps its sign.
 __device__ __forceinline__ double mdiv_try(double a, double b, double y, bool& ok) {
   const double q0 = a * y;
-  const double r = __fma_rn(-q0, b, a);
-  const double q1 = __fma_rn(r, y, q0);
   const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu;
   const unsigned hy = (unsigned)__double2hiint(y) & 0x7fffffffu;
-  const bool zero = a == 0.0;
-  ok = ok && (hy - (623u << 20) < (800u << 20)) && ((ha - (523u << 20) < (1000u << 20)) || zero);
-  return zero ? q0 : q1;
+  ok = ok & (hy - (623u << 20) < (800u << 20)) &
+       ((ha - (523u << 20) < (1000u << 20)) | ((ha | (unsigned)__double2loint(a)) == 0u));
+  return __fma_rn(-__fma_rn(q0, b, -a), y, q0);
 }
 
 __device__ __forceinline__ bool is_null(const GridDev& G, int i1, int i2, int i3) {
@@ -3231,7 +3230,7 @@ __device__ __forceinline__ void dt_cell(const GridDev& G, long long mk, int i1, 
 
 template <bool UNIT, int MODE /*0 gridrates, 1 maxcfl*/>
 __device__ __forceinline__ void b_dt_reduce(const GridDev& G, const Blocks& B, unsigned long long* acc /*3*LSP*/,
-                                                        const double* dtp, const VB vb) {
+                                            const double* dtp, const VB vb, double* part = nullptr) {
   const Dims d = G.d;
   const int s = threadIdx.y;
   const int lane = threadIdx.x;
@@ -3265,24 +3264,71 @@ __device__ __forceinline__ void b_dt_reduce(const GridDev& G, const Blocks& B, u
   }
   if (lane == 0) {
     if (MODE == 0) {
-      atomicMax(acc + s, (unsigned long long)__double_as_longlong(g1));
-      atomicMax(acc + LSP + s, (unsigned long long)__double_as_longlong(g2));
-      atomicMax(acc + 2 * LSP + s, (unsigned long long)__double_as_longlong(g3));
+      if (part) {
+        part[(long long)s * vb.gx + vb.bx] = g1;
+        part[(long long)(LSP + s) * vb.gx + vb.bx] = g2;
+        part[(long long)(2 * LSP + s) * vb.gx + vb.bx] = g3;
+      } else {
+        atomicMax(acc + s, (unsigned long long)__double_as_longlong(g1));
+        atomicMax(acc + LSP + s, (unsigned long long)__double_as_longlong(g2));
+        atomicMax(acc + 2 * LSP + s, (unsigned long long)__double_as_longlong(g3));
+      }
     } else {
       atomicMax(acc, (unsigned long long)__double_as_longlong(g1));
     }
   }
 }
 
-template <bool UNIT, int MODE /*0 gridrates, 1 maxcfl*/>
-__global__ void __launch_bounds__(32 * LSP, GEM_DT_MINB) k_dt_reduce(GridDev G, Blocks B, unsigned long long* acc /*3*LSP*/,
-                                                        const double* dtp) {
-  b_dt_reduce<UNIT, MODE>(G, B, acc, dtp, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
+// Max CFL over the grid (acc[0]).
+template <bool UNIT>
+__global__ void __launch_bounds__(32 * LSP, GEM_DT_MINB) k_maxcfl(GridDev G, Blocks B, unsigned long long* acc,
+                                                                  const double* dtp) {
+  b_dt_reduce<UNIT, 1>(G, B, acc, dtp, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
+}
+
+// The time step (temporal_mpi.f90:86-167).  Each block stores its 3*LSP maxima, and the block
+// that finishes last (count) reduces them: three atomics a warp on 21 neighbouring addresses
+// cost more than the rates of a small grid, as did a launch that only finished the reduction
+// (64x8x6: 8.5 us in three launches, 7.2 in one).  384x192x192: 0.93 -> 0.86 ms, 0.62 of the copy
+// peak by the 31 doubles a cell it needs.  count is zero between calls.
+template <bool UNIT>
+__global__ void __launch_bounds__(32 * LSP, GEM_DT_MINB) k_dt_calc(GridDev G, Blocks B, double* part,
+                                                                   unsigned long long* count, double tcfl,
+                                                                   double* dt_out) {
+  b_dt_reduce<UNIT, 0>(G, B, nullptr, nullptr, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x}, part);
+  __shared__ bool last;
+  __shared__ double inv[LSP];
+  const int s = threadIdx.y, lane = threadIdx.x, nb = gridDim.x;
+  __syncthreads();
+  if (lane == 0 && s == 0) {
+    __threadfence();  // the block's stores, ordered by the barrier, before its count
+    last = atomicAdd(count, 1ull) == (unsigned long long)nb - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double m = 0.0;
+  for (int d = 0; d < 3; ++d) {
+    const double* p = part + (long long)(d * LSP + s) * nb;
+    double g = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < nb; b += 32) g = fmax_f(__ldcg(p + b), g);
+    for (int o = 16; o > 0; o >>= 1) g = fmax_f(g, __shfl_xor_sync(0xffffffffu, g, o));
+    const double r = 1.0 / fmax_f(g, 1e-10);  // the smallest of 1/rate, the rates at least 1e-10
+    m = (d == 0 || r < m) ? r : m;
+  }
+  if (lane == 0) inv[s] = m;
+  __syncthreads();
+  if (lane == 0 && s == 0) {
+    for (int q = 1; q < LSP; ++q) m = fmin_f(inv[q], m);
+    *dt_out = fmax_f(tcfl * m, 1e-6);
+    *count = 0;
+  }
 }
 
 
 // Per-x3-plane partial maxima of the dt rates (block i3 covers the plane's x1 rows):
-// part[(i3-1)*3*LSP + slot], slot as in k_dt_reduce.  Every slot of every plane is written.
+// part[(i3-1)*3*LSP + slot], slot as in b_dt_reduce.  Every slot of every plane is written.
 template <bool UNIT>
 __global__ void __launch_bounds__(32 * LSP) k_dt_reduce_planes(GridDev G, Blocks B, double* part) {
   const Dims d = G.d;
@@ -3321,7 +3367,7 @@ __global__ void __launch_bounds__(32 * LSP) k_dt_reduce_planes(GridDev G, Blocks
   }
 }
 
-// max over the planes per slot, then the k_dt_finalize formula (one warp)
+// max over the planes per slot, then k_dt_calc's formula for the step (one warp)
 __global__ void k_dt_finalize_planes(const double* part, int nplane, double tcfl, double* dt_out) {
   const int lane = threadIdx.x;
   double m = 0.0;
@@ -3333,17 +3379,6 @@ __global__ void k_dt_finalize_planes(const double* part, int nplane, double tcfl
     if (q == 0 || inv < m) m = inv;
   }
   if (lane == 0) *dt_out = fmax_f(tcfl * m, 1e-6);
-}
-
-__global__ void k_dt_finalize(const unsigned long long* acc, double tcfl, double* dt_out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double m = 0.0;
-  for (int q = 0; q < 3 * LSP; ++q) {
-    const double gr = fmax_f(__longlong_as_double((long long)acc[q]), 1e-10);
-    const double inv = 1.0 / gr;
-    if (q == 0 || inv < m) m = inv;
-  }
-  *dt_out = fmax_f(tcfl * m, 1e-6);
 }
 
 __global__ void k_maxcfl_finalize(const unsigned long long* acc, double* out) {
