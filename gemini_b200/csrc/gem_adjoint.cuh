@@ -26,6 +26,7 @@ namespace gemk {
 
 // faces 1 and lx1+1 of a vs1i face array from the (LSP, lx3, lx2) boundary arrays
 __global__ void ka_set_faces(Dims d, const double* __restrict__ lo, const double* __restrict__ hi, double* v1i) {
+  step_entry();
   const long long ncol = (long long)d.lx2 * d.lx3;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ncol * LSP;
        t += (long long)gridDim.x * blockDim.x) {
@@ -43,6 +44,7 @@ __global__ void ka_replay_in(Dims d, const double* __restrict__ ns, const double
                              const double* __restrict__ vs2, const double* __restrict__ vs3,
                              const double* __restrict__ Ts, double* __restrict__ W, double* __restrict__ rv,
                              double* __restrict__ re) {
+  step_entry();
   const int s = blockIdx.y;
   const long long F = LSP * d.ng, b = s * d.ng;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < d.ng; q += (long long)gridDim.x * blockDim.x) {
@@ -61,6 +63,7 @@ __global__ void ka_replay_in(Dims d, const double* __restrict__ ns, const double
 // What an out-of-place sweep of the three fields leaves unwritten, copied: every ghost cell,
 // and the electrons of the first two fields.  A warp per x1 row.
 __global__ void ka_rest_copy(GridDev G, const double* __restrict__ C, double* __restrict__ Cn) {
+  step_entry();
   const Dims d = G.d;
   const int X2 = d.lx2 + 4, X3 = d.lx3 + 4;
   const int nrow = X2 * X3 * 3 * LSP;
@@ -126,6 +129,7 @@ __device__ __forceinline__ void for_rows_s(const Dims& d, Body body) {
 // electrons the ion sum; ghosts 1e-5) and T after rhoe2T + clean_param(3) (ghosts 100).
 // F: the swept stage (n | rv | re blocks).
 __global__ void ka_post_fwd(GridDev G, const double* __restrict__ F, double* nout, double* Tpre) {
+  step_entry();
   const Dims d = G.d;
   const long long ng = d.ng;
   const double* re = F + 2 * LSP * ng;
@@ -160,6 +164,7 @@ __global__ void ka_post_fwd(GridDev G, const double* __restrict__ F, double* nou
 // ns, rv, vs1, Ts written into B are the forward step's bits. Ghost cells get the swept n and
 // rv, which k_ghost_epilogue then turns into the forward's ghost values.
 __global__ void ka_finish_fwd(GridDev G, const double* __restrict__ F, Blocks B) {
+  step_entry();
   const Dims d = G.d;
   const long long ng = d.ng;
   const double* fn = F;
@@ -204,6 +209,7 @@ __global__ void ka_finish_fwd(GridDev G, const double* __restrict__ F, Blocks B)
 // The two boundary faces of every x1 column (the state's lo / hi), read from a face array:
 // the inverse of ka_set_faces.
 __global__ void ka_get_faces(Dims d, const double* __restrict__ v1i, double* lo, double* hi) {
+  step_entry();
   const long long ncol = (long long)d.lx2 * d.lx3;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ncol * LSP;
        t += (long long)gridDim.x * blockDim.x) {
@@ -223,6 +229,7 @@ __global__ void __launch_bounds__(256) ka_post_vjp(GridDev G, const double* __re
                                                    const double* __restrict__ nbo, const double* __restrict__ vbo,
                                                    const double* __restrict__ TPb, const double* __restrict__ NDb,
                                                    double* C) {
+  step_entry();
   const Dims d = G.d;
   const long long ng = d.ng;
   const double* rv = F + LSP * ng;
@@ -288,6 +295,7 @@ __global__ void __launch_bounds__(256) ka_post_vjp(GridDev G, const double* __re
 // Adjoint of the periodic x3 self-wrap (mpihalo.f90:147-151) on n, rv, re: rows 1:lx2,
 // every x1.  The ghost layers' cotangents move to their source layers.
 __global__ void ka_wrap3_vjp(GridDev G, double* C) {
+  step_entry();
   const Dims d = G.d;
   const int n1 = d.lx1 + 4;
   const long long nrow = (long long)n1 * d.lx2;
@@ -315,6 +323,7 @@ __global__ void ka_wrap3_vjp(GridDev G, double* C) {
 // re, over every cell of the other two directions (advec.f90:83-132).
 template <int DIM>
 __global__ void ka_copy_vjp(GridDev G, double* C) {
+  step_entry();
   const Dims d = G.d;
   const int na = d.lx1 + 4;
   const int nb = (DIM == 2) ? d.lx3 + 4 : d.lx2 + 4;
@@ -343,6 +352,7 @@ __global__ void ka_copy_vjp(GridDev G, double* C) {
 // nsp -- keep C's value.
 template <int DIM>
 __global__ void ka_frame_copy(GridDev G, const double* __restrict__ C, double* Cn) {
+  step_entry();
   const Dims d = G.d;
   const long long ng = d.ng;
   const int X2 = d.lx2 + 4, X3 = d.lx3 + 4;
@@ -386,6 +396,7 @@ __global__ void ka_x1bc_vjp(GridDev G, const double* __restrict__ ns, const doub
                             const double* __restrict__ Ts, const double* __restrict__ lo,
                             const double* __restrict__ hi, double* C, double* vext, double* lob, double* hib,
                             const double* __restrict__ ttb, double* Ttop_bar) {
+  step_entry();
   const Dims d = G.d;
   const long long ng = d.ng;
   const long long ncol = (long long)d.lx2 * d.lx3;
@@ -511,6 +522,7 @@ __global__ void ka_conv_vjp(GridDev G, const double* __restrict__ ns, const doub
                             const double* __restrict__ v1ib, const double* __restrict__ lob_out,
                             const double* __restrict__ hib_out, const double* __restrict__ vext, double* nsb,
                             double* vs1b, double* Tsb) {
+  step_entry();
   const Dims d = G.d;
   const long long ng = d.ng;
   const long long ncol = (long long)d.lx2 * d.lx3;
@@ -667,14 +679,14 @@ int gem_step_vjp_replay_dev(const gem_cfg* cfg, const gem_grid* g, const gem_wor
   const size_t FB = sizeof(double) * F;
   double* S0 = A->ST;
   // ---------------- forward replay
-  ka_replay_in<<<dim3(grid_for(d.ng, 256), LSP), 256, 0, st>>>(d, ns, vs1, vs2, vs3, Ts, WF, S0 + F, S0 + 2 * F);
+  step_launch(ka_replay_in, dim3(grid_for(d.ng, 256), LSP), 256, 0, st, d, ns, vs1, vs2, vs3, Ts, WF, S0 + F, S0 + 2 * F);
   GEM_LAUNCHED("ka_replay_in");
-  ka_set_faces<<<grid_for(ncol * LSP, 256), 256, 0, st>>>(d, v1i_lo, v1i_hi, A->VP);
+  step_launch(ka_set_faces, grid_for(ncol * LSP, 256), 256, 0, st, d, v1i_lo, v1i_hi, A->VP);
   GEM_LAUNCHED("ka_set_faces");
   Blocks B = blocks(g, WF, S0 + F);  // rv, re straight into stage 0
   if ((rc = launch_ghost_fill(g, B, A->VP, LSP, false, st))) return rc;
   if (G.flagper) {
-    k_halo_wrap<<<grid_for((long long)(d.lx1 + 4) * d.lx2 * LSP, 256), 256, 0, st>>>(G, B, 1);
+    step_launch(k_halo_wrap, grid_for((long long)(d.lx1 + 4) * d.lx2 * LSP, 256), 256, 0, st, G, B, 1);
     GEM_LAUNCHED("k_halo_wrap");
   }
   GEM_CUDA(cudaMemcpyAsync(S0, WF, FB, cudaMemcpyDeviceToDevice, st));
@@ -689,7 +701,7 @@ int gem_step_vjp_replay_dev(const gem_cfg* cfg, const gem_grid* g, const gem_wor
   for (int q = 0; q < 3; ++q) {
     double* Sin = Sx[q];
     double* So = Sx[q + 1];
-    ka_rest_copy<<<ngb, 256, 0, st>>>(G, Sin, So);
+    step_launch(ka_rest_copy, ngb, 256, 0, st, G, Sin, So);
     GEM_LAUNCHED("ka_rest_copy");
     SweepTri T;
     T.a.G = G;
@@ -703,14 +715,14 @@ int gem_step_vjp_replay_dev(const gem_cfg* cfg, const gem_grid* g, const gem_wor
     if ((rc = launch_sweep_tri(g, dims[q], T, st))) return rc;
     if (q == 1 && G.flagper) {  // halo_allparams self-wrap between the x1 and x2 sweeps
       Blocks wb = blocks(g, So, So + F);
-      k_halo_wrap<<<grid_for((long long)(d.lx1 + 4) * d.lx2 * LSP, 256), 256, 0, st>>>(G, wb, 0);
+      step_launch(k_halo_wrap, grid_for((long long)(d.lx1 + 4) * d.lx2 * LSP, 256), 256, 0, st, G, wb, 0);
       GEM_LAUNCHED("k_halo_wrap");
     }
   }
   // the post-sweep values the diffusion adjoint needs (WF's state copy is dead now)
   double* NO = WF;
   double* TP = WF + F;
-  ka_post_fwd<<<ngb, 256, 0, st>>>(G, Sx[3], NO, TP);
+  step_launch(ka_post_fwd, ngb, 256, 0, st, G, Sx[3], NO, TP);
   GEM_LAUNCHED("ka_post_fwd");
   return GEM_OK;
 }
@@ -728,12 +740,12 @@ int gem_step_vjp_finish_dev(const gem_cfg* cfg, const gem_grid* g, gem_work* w, 
   const long long ncol = (long long)d.lx2 * d.lx3;
   Blocks B = blocks(g, fluidvars, fluidauxvars);
   // the x2 sweep's epilogue from the replay's last stage, then the rest of gem_fluid_adv_dev
-  ka_finish_fwd<<<grid_for(d.ng, 256), 256, 0, st>>>(G, A->ST + 9 * A->F, B);
+  step_launch(ka_finish_fwd, grid_for(d.ng, 256), 256, 0, st, G, A->ST + 9 * A->F, B);
   GEM_LAUNCHED("ka_finish_fwd");
-  k_ghost_epilogue<<<grid_for(ghost_cells(d), 256), 256, 0, st>>>(G, B);
+  step_launch(k_ghost_epilogue<false>, grid_for(ghost_cells(d), 256), 256, 0, st, G, B);
   GEM_LAUNCHED("k_ghost_epilogue");
   if (G.has_null && (G.gridflag == 0 || G.gridflag == 1)) {
-    k_clean_vel_edges<<<grid_for(ncol * LSP, 128), 128, 0, st>>>(G, fluidvars + LSP * d.ng);
+    step_launch(k_clean_vel_edges, grid_for(ncol * LSP, 128), 128, 0, st, G, fluidvars + LSP * d.ng);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
   DiffArgs da;
@@ -751,7 +763,7 @@ int gem_step_vjp_finish_dev(const gem_cfg* cfg, const gem_grid* g, gem_work* w, 
   if ((rc = launch_diffusion(g, da, st))) return rc;
   // the boundary faces the forward's x1 sweep stores for the next step: the replay's x1
   // interface velocities there (the same formulas, advec.f90:170-196)
-  ka_get_faces<<<grid_for(ncol * LSP, 256), 256, 0, st>>>(d, A->V1, v1i_lo, v1i_hi);
+  step_launch(ka_get_faces, grid_for(ncol * LSP, 256), 256, 0, st, d, A->V1, v1i_lo, v1i_hi);
   GEM_LAUNCHED("ka_get_faces");
   return GEM_OK;
 }
@@ -803,21 +815,21 @@ int gem_step_vjp_backward_dev(const gem_cfg* cfg, const gem_grid* g, const gem_w
   }
   double* C = A->CA;
   double* Cn = A->CB;
-  ka_post_vjp<<<ngb, 256, 0, st>>>(G, Sx[3], ns_bar_out, vs1_bar_out, TPB, NDB, C);
+  step_launch(ka_post_vjp, ngb, 256, 0, st, G, Sx[3], ns_bar_out, vs1_bar_out, TPB, NDB, C);
   GEM_LAUNCHED("ka_post_vjp");
   const long long nvf = (long long)LSP * nf1(d);  // one field's vs1i cotangent slice
   GEM_CUDA(cudaMemsetAsync(A->VB, 0, sizeof(double) * 3 * nvf, st));
   for (int q = 2; q >= 0; --q) {
     if (q == 1 && G.flagper) {
-      ka_wrap3_vjp<<<grid_for((long long)(d.lx1 + 4) * d.lx2 * 3 * LSP, 256), 256, 0, st>>>(G, C);
+      step_launch(ka_wrap3_vjp, grid_for((long long)(d.lx1 + 4) * d.lx2 * 3 * LSP, 256), 256, 0, st, G, C);
       GEM_LAUNCHED("ka_wrap3_vjp");
     }
     if (dims[q] == 1)
-      ka_frame_copy<1><<<ngb, 256, 0, st>>>(G, C, Cn);
+      step_launch(ka_frame_copy<1>, ngb, 256, 0, st, G, C, Cn);
     else if (dims[q] == 2)
-      ka_frame_copy<2><<<ngb, 256, 0, st>>>(G, C, Cn);
+      step_launch(ka_frame_copy<2>, ngb, 256, 0, st, G, C, Cn);
     else
-      ka_frame_copy<3><<<ngb, 256, 0, st>>>(G, C, Cn);
+      step_launch(ka_frame_copy<3>, ngb, 256, 0, st, G, C, Cn);
     GEM_LAUNCHED("ka_frame_copy");
     // the three fields in one launch; x1 also gives each field's vs1i cotangent (its own
     // slice of VB, summed by ka_conv_vjp); the x2/x3 velocities are fixed
@@ -841,18 +853,18 @@ int gem_step_vjp_backward_dev(const gem_cfg* cfg, const gem_grid* g, const gem_w
   }
   // the ghost fill's x3 pass: edge copies, or the periodic self-wrap
   if (G.flagper) {
-    ka_wrap3_vjp<<<grid_for((long long)(d.lx1 + 4) * d.lx2 * 3 * LSP, 256), 256, 0, st>>>(G, C);
+    step_launch(ka_wrap3_vjp, grid_for((long long)(d.lx1 + 4) * d.lx2 * 3 * LSP, 256), 256, 0, st, G, C);
     GEM_LAUNCHED("ka_wrap3_vjp");
   } else {
-    ka_copy_vjp<3><<<grid_for((long long)(d.lx1 + 4) * (d.lx2 + 4) * 3 * LSP, 256), 256, 0, st>>>(G, C);
+    step_launch(ka_copy_vjp<3>, grid_for((long long)(d.lx1 + 4) * (d.lx2 + 4) * 3 * LSP, 256), 256, 0, st, G, C);
     GEM_LAUNCHED("ka_copy_vjp<3>");
   }
-  ka_copy_vjp<2><<<grid_for((long long)(d.lx1 + 4) * (d.lx3 + 4) * 3 * LSP, 256), 256, 0, st>>>(G, C);
+  step_launch(ka_copy_vjp<2>, grid_for((long long)(d.lx1 + 4) * (d.lx3 + 4) * 3 * LSP, 256), 256, 0, st, G, C);
   GEM_LAUNCHED("ka_copy_vjp<2>");
-  ka_x1bc_vjp<<<grid_for(ncol * LSP, 128), 128, 0, st>>>(G, ns, vs1, Ts, v1i_lo, v1i_hi, C, A->vext, lo_bar, hi_bar,
+  step_launch(ka_x1bc_vjp, grid_for(ncol * LSP, 128), 128, 0, st, G, ns, vs1, Ts, v1i_lo, v1i_hi, C, A->vext, lo_bar, hi_bar,
                                                     Ttop_bar ? A->ttb : nullptr, Ttop_bar);
   GEM_LAUNCHED("ka_x1bc_vjp");
-  ka_conv_vjp<<<ngb, 256, 0, st>>>(G, ns, vs1, Ts, C, A->VB, lo_bar_out, hi_bar_out, A->vext, ns_bar, vs1_bar,
+  step_launch(ka_conv_vjp, ngb, 256, 0, st, G, ns, vs1, Ts, C, A->VB, lo_bar_out, hi_bar_out, A->vext, ns_bar, vs1_bar,
                                    Ts_bar);
   GEM_LAUNCHED("ka_conv_vjp");
   return GEM_OK;

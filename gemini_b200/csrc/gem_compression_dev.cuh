@@ -8,24 +8,29 @@ namespace gemk {
 
 __global__ void kc_artvisc(gemc::View v, long long n, const double* __restrict__ ns,
                            const double* __restrict__ vs1, double* __restrict__ Q) {
+  step_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
     gemc::artvisc(v, t, ns, vs1, Q);
 }
 __global__ void kc_rk2_x1(gemc::View v, long long n, double* vs1) {
+  step_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
     gemc::rk2_x1(v, t, vs1);
 }
 __global__ void kc_rk2_x2(gemc::View v, long long n, double* vs1, double* vs2, double* vs3) {
+  step_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
     gemc::rk2_x2(v, t, vs1, vs2, vs3);
 }
 __global__ void kc_rk2_x3(gemc::View v, long long n, double* vs1, double* vs2, double* vs3) {
+  step_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
     gemc::rk2_x3(v, t, vs1, vs2, vs3);
 }
 __global__ void kc_compression(gemc::View v, long long n, const double* __restrict__ vs1,
                                const double* __restrict__ vs2, const double* __restrict__ vs3,
                                const double* __restrict__ Q, double* rhoes, const double* __restrict__ dtp) {
+  step_entry();
   const double dt = *dtp;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
     gemc::cmp(v, t, vs1, vs2, vs3, Q, rhoes, dt);
@@ -43,6 +48,7 @@ __global__ void kc_compression(gemc::View v, long long n, const double* __restri
 // a cell and species needs).
 template <bool UNIT>
 __global__ void kc_compress_T(GridDev G, Blocks B, double* __restrict__ Q, const double* __restrict__ dtp) {
+  step_entry();
   const Dims d = G.d;
   const double dt = *dtp;
   const int s = blockIdx.y;
@@ -142,7 +148,7 @@ int gem_vnricht_artvisc_dev(const gem_grid* g, const double* fluidvars, double* 
   if (check_grid(g) || !fluidvars || !Q) return set_err(GEM_EINVAL, "null argument");
   const gemc::View v = gemk::cmp_view(g);
   const long long n = gemc::ncell(v) * LSP;
-  gemk::kc_artvisc<<<grid_for(n, 256), 256, 0, S(stream)>>>(v, n, fluidvars, fluidvars + LSP * v.ng, Q);
+  step_launch(gemk::kc_artvisc, grid_for(n, 256), 256, 0, S(stream), v, n, fluidvars, fluidvars + LSP * v.ng, Q);
   GEM_LAUNCHED("kc_artvisc");
   return GEM_OK;
 }
@@ -155,14 +161,14 @@ int gem_rk2_global_boundary_allspec_dev(const gem_grid* g, double* fluidvars, vo
   double* vs3 = fluidvars + 3 * LSP * v.ng;
   cudaStream_t st = S(stream);
   const long long n1 = (long long)(v.lx2 + 4) * (v.lx3 + 4) * LSP;
-  gemk::kc_rk2_x1<<<grid_for(n1, 256), 256, 0, st>>>(v, n1, vs1);
+  step_launch(gemk::kc_rk2_x1, grid_for(n1, 256), 256, 0, st, v, n1, vs1);
   GEM_LAUNCHED("kc_rk2_x1");
   const long long n2 = (long long)(v.lx1 + 4) * (v.lx3 + 4) * LSP * 3;
-  gemk::kc_rk2_x2<<<grid_for(n2, 256), 256, 0, st>>>(v, n2, vs1, vs2, vs3);
+  step_launch(gemk::kc_rk2_x2, grid_for(n2, 256), 256, 0, st, v, n2, vs1, vs2, vs3);
   GEM_LAUNCHED("kc_rk2_x2");
   if (!v.flagper) {
     const long long n3 = (long long)(v.lx1 + 4) * (v.lx2 + 4) * LSP * 3;
-    gemk::kc_rk2_x3<<<grid_for(n3, 256), 256, 0, st>>>(v, n3, vs1, vs2, vs3);
+    step_launch(gemk::kc_rk2_x3, grid_for(n3, 256), 256, 0, st, v, n3, vs1, vs2, vs3);
     GEM_LAUNCHED("kc_rk2_x3");
   }
   return GEM_OK;
@@ -173,7 +179,7 @@ int gem_compression_dev(const gem_grid* g, const double* fluidvars, double* flui
   if (check_grid(g) || !fluidvars || !fluidauxvars || !Q || !dt) return set_err(GEM_EINVAL, "null argument");
   const gemc::View v = gemk::cmp_view(g);
   const long long n = gemc::ncell(v) * LSP;
-  gemk::kc_compression<<<grid_for(n, 256), 256, 0, S(stream)>>>(v, n, fluidvars + LSP * v.ng,
+  step_launch(gemk::kc_compression, grid_for(n, 256), 256, 0, S(stream), v, n, fluidvars + LSP * v.ng,
                                                                   fluidvars + 2 * LSP * v.ng,
                                                                   fluidvars + 3 * LSP * v.ng, Q,
                                                                   fluidauxvars + LSP * v.ng, dt);

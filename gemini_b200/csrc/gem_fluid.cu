@@ -80,6 +80,23 @@ unsigned grid_for(long long n, int threads, int per_sm = 8) {
   return (unsigned)b;
 }
 
+// Launch of a kernel that begins with step_entry(): it may start before the previous kernel of
+// the stream has completed, and waits there.
+template <class... KArgs, class... Args>
+void step_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kern, KArgs(args)...);
+}
+
 // blocks of the dt and CFL reductions: a block per x1 row up to the four an SM holds (eight, a
 // second partial wave: 96x32x32 20.4 us against 17.3; the same at 384x192x192)
 unsigned dt_blocks(const Dims& d) {
@@ -202,12 +219,12 @@ int launch_sweep_t(const gem_grid* g, SweepArgs a, int nsp, cudaStream_t st) {
     // one warp per (x1 column, species)
     dim3 grid(d.lx2, d.lx3);
     if (FUSED && a.nsB) {
-      if (g->dev.unit) k_sweep_x1<true, FUSED, FUSED><<<grid, block, 0, st>>>(a);
-      else k_sweep_x1<false, FUSED, FUSED><<<grid, block, 0, st>>>(a);
+      if (g->dev.unit) step_launch(k_sweep_x1<true, FUSED, FUSED>, grid, block, 0, st, a);
+      else step_launch(k_sweep_x1<false, FUSED, FUSED>, grid, block, 0, st, a);
     } else if (g->dev.unit) {
-      k_sweep_x1<true, FUSED><<<grid, block, 0, st>>>(a);
+      step_launch(k_sweep_x1<true, FUSED>, grid, block, 0, st, a);
     } else {
-      k_sweep_x1<false, FUSED><<<grid, block, 0, st>>>(a);
+      step_launch(k_sweep_x1<false, FUSED>, grid, block, 0, st, a);
     }
     GEM_LAUNCHED("k_sweep_x1");
     return GEM_OK;
@@ -217,22 +234,22 @@ int launch_sweep_t(const gem_grid* g, SweepArgs a, int nsp, cudaStream_t st) {
   if (DIM == 3 && FUSED) {  // periodicity as a template parameter
     const bool per = g->dev.flagper != 0;
     if (g->dev.unit) {
-      if (per) k_sweep_march<3, true, true, 1><<<grid, block, 0, st>>>(a);
-      else k_sweep_march<3, true, true, 0><<<grid, block, 0, st>>>(a);
+      if (per) step_launch(k_sweep_march<3, true, true, 1>, grid, block, 0, st, a);
+      else step_launch(k_sweep_march<3, true, true, 0>, grid, block, 0, st, a);
     } else {
       const bool inv = g->dev.c3 == 0;
-      if (per && inv) k_sweep_march<3, false, true, 1, false, true><<<grid, block, 0, st>>>(a);
-      else if (per) k_sweep_march<3, false, true, 1><<<grid, block, 0, st>>>(a);
-      else if (inv) k_sweep_march<3, false, true, 0, false, true><<<grid, block, 0, st>>>(a);
-      else k_sweep_march<3, false, true, 0><<<grid, block, 0, st>>>(a);
+      if (per && inv) step_launch(k_sweep_march<3, false, true, 1, false, true>, grid, block, 0, st, a);
+      else if (per) step_launch(k_sweep_march<3, false, true, 1>, grid, block, 0, st, a);
+      else if (inv) step_launch(k_sweep_march<3, false, true, 0, false, true>, grid, block, 0, st, a);
+      else step_launch(k_sweep_march<3, false, true, 0>, grid, block, 0, st, a);
     }
     GEM_LAUNCHED("k_sweep_march");
     return GEM_OK;
   }
   if (g->dev.unit)
-    k_sweep_march<DIM == 3 ? 3 : 2, true, FUSED><<<grid, block, 0, st>>>(a);
+    step_launch(k_sweep_march<DIM == 3 ? 3 : 2, true, FUSED>, grid, block, 0, st, a);
   else
-    k_sweep_march<DIM == 3 ? 3 : 2, false, FUSED><<<grid, block, 0, st>>>(a);
+    step_launch(k_sweep_march<DIM == 3 ? 3 : 2, false, FUSED>, grid, block, 0, st, a);
   GEM_LAUNCHED("k_sweep_march");
   return GEM_OK;
 }
@@ -255,11 +272,11 @@ int launch_sweep_tri(const gem_grid* g, int dim, const SweepTri& T, cudaStream_t
   const dim3 block(32, LSP);
   if (dim == 1) {
     auto kern = u ? k_sweep_tri_x1<true> : k_sweep_tri_x1<false>;
-    kern<<<dim3(d.lx2, d.lx3, 3), block, 0, st>>>(T);
+    step_launch(kern, dim3(d.lx2, d.lx3, 3), block, 0, st, T);
   } else {
     auto kern = dim == 3 ? (u ? k_sweep_tri<3, true> : k_sweep_tri<3, false>)
                          : (u ? k_sweep_tri<2, true> : k_sweep_tri<2, false>);
-    kern<<<dim3((d.lx1 + 31) / 32, dim == 3 ? d.lx2 : d.lx3, 3 * sweep_parts(d, dim)), block, 0, st>>>(T);
+    step_launch(kern, dim3((d.lx1 + 31) / 32, dim == 3 ? d.lx2 : d.lx3, 3 * sweep_parts(d, dim)), block, 0, st, T);
   }
   GEM_LAUNCHED("k_sweep_tri");
   return GEM_OK;
@@ -273,16 +290,16 @@ int launch_ghost_fill(const gem_grid* g, Blocks B, const double* vs1i, int lsp, 
   const long long nrow2 = (long long)(d.lx1 + 4) * (d.lx3 + 4) * lsp;
   const long long nrow3 = (long long)(d.lx1 + 4) * (d.lx2 + 4) * lsp;
   if (fused) {
-    k_ghost_x1<true><<<grid_for(ncol, 128), 128, 0, st>>>(G, B, vs1i, lsp);
-    k_ghost_x2<true><<<grid_for(nrow2, 128), 128, 0, st>>>(G, B, lsp);
+    step_launch(k_ghost_x1<true>, grid_for(ncol, 128), 128, 0, st, G, B, vs1i, lsp);
+    step_launch(k_ghost_x2<true>, grid_for(nrow2, 128), 128, 0, st, G, B, lsp);
     if (G.flagper)
-      k_ghost_x3<true, true><<<grid_for(nrow3, 128), 128, 0, st>>>(G, B, lsp);
+      step_launch(k_ghost_x3<true, true>, grid_for(nrow3, 128), 128, 0, st, G, B, lsp);
     else
-      k_ghost_x3<true, false><<<grid_for(nrow3, 128), 128, 0, st>>>(G, B, lsp);
+      step_launch(k_ghost_x3<true, false>, grid_for(nrow3, 128), 128, 0, st, G, B, lsp);
   } else {
-    k_ghost_x1<false><<<grid_for(ncol, 128), 128, 0, st>>>(G, B, vs1i, lsp);
-    k_ghost_x2<false><<<grid_for(nrow2, 128), 128, 0, st>>>(G, B, lsp);
-    if (!G.flagper) k_ghost_x3<false, false><<<grid_for(nrow3, 128), 128, 0, st>>>(G, B, lsp);
+    step_launch(k_ghost_x1<false>, grid_for(ncol, 128), 128, 0, st, G, B, vs1i, lsp);
+    step_launch(k_ghost_x2<false>, grid_for(nrow2, 128), 128, 0, st, G, B, lsp);
+    if (!G.flagper) step_launch(k_ghost_x3<false, false>, grid_for(nrow3, 128), 128, 0, st, G, B, lsp);
   }
   GEM_LAUNCHED("ghost fill");
   return GEM_OK;
@@ -362,7 +379,7 @@ int launch_diffusion_lu(const gem_grid* g, DiffArgs a, cudaStream_t st) {
     const size_t sm = luc_bytes(d.lx1) * cb;
     auto kern = g->dev.unit ? k_diffusion_col<true> : k_diffusion_col<false>;
     if (sm > 48 * 1024) GEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    kern<<<(unsigned)(ng * LSP), 32 * warps, sm, st>>>(a, cb);
+    step_launch(kern, (unsigned)(ng * LSP), 32 * warps, sm, st, a, cb);
     GEM_LAUNCHED("k_diffusion_col");
     return GEM_OK;
   }
@@ -370,7 +387,7 @@ int launch_diffusion_lu(const gem_grid* g, DiffArgs a, cudaStream_t st) {
   const bool few = nblk <= (long long)num_sms() * LU_MINB_FEW;
   auto kern = g->dev.unit ? (few ? k_diffusion_lu<true, LU_MINB_FEW> : k_diffusion_lu<true, LU_MINB>)
                           : (few ? k_diffusion_lu<false, LU_MINB_FEW> : k_diffusion_lu<false, LU_MINB>);
-  kern<<<(unsigned)nblk, 32 * LU_WPB, 0, st>>>(a);
+  step_launch(kern, (unsigned)nblk, 32 * LU_WPB, 0, st, a);
   GEM_LAUNCHED("k_diffusion_lu");
   return GEM_OK;
 }
@@ -398,11 +415,11 @@ int launch_sweep_vjp_march(const gem_grid* g, int dim, const SweepVjpFields& FS,
   const long long nl = (long long)d.lx1 * ((dim == 2) ? d.lx3 : d.lx2);
   const unsigned nb = grid_for(nl * nseg * FS.nfs, 256, 8);
   if (g->dev.unit) {
-    if (dim == 2) k_sweep_vjp_march<2, true><<<nb, 256, 0, st>>>(a, FS, nseg);
-    else k_sweep_vjp_march<3, true><<<nb, 256, 0, st>>>(a, FS, nseg);
+    if (dim == 2) step_launch(k_sweep_vjp_march<2, true>, nb, 256, 0, st, a, FS, nseg);
+    else step_launch(k_sweep_vjp_march<3, true>, nb, 256, 0, st, a, FS, nseg);
   } else {
-    if (dim == 2) k_sweep_vjp_march<2, false><<<nb, 256, 0, st>>>(a, FS, nseg);
-    else k_sweep_vjp_march<3, false><<<nb, 256, 0, st>>>(a, FS, nseg);
+    if (dim == 2) step_launch(k_sweep_vjp_march<2, false>, nb, 256, 0, st, a, FS, nseg);
+    else step_launch(k_sweep_vjp_march<3, false>, nb, 256, 0, st, a, FS, nseg);
   }
   GEM_LAUNCHED("k_sweep_vjp_march");
   return GEM_OK;
@@ -427,9 +444,9 @@ int launch_sweep_vjp_x1(const gem_grid* g, const SweepVjpFields& FS, const doubl
   const long long nwarp = (long long)d.lx2 * d.lx3 * FS.nfs;
   const unsigned nb = (unsigned)std::min<long long>((nwarp + 7) / 8, (long long)num_sms() * 8);
   if (g->dev.unit)
-    k_sweep_vjp_x1<true><<<nb, 256, 0, st>>>(a, FS);
+    step_launch(k_sweep_vjp_x1<true>, nb, 256, 0, st, a, FS);
   else
-    k_sweep_vjp_x1<false><<<nb, 256, 0, st>>>(a, FS);
+    step_launch(k_sweep_vjp_x1<false>, nb, 256, 0, st, a, FS);
   GEM_LAUNCHED("k_sweep_vjp_x1");
   return GEM_OK;
 }
@@ -480,7 +497,7 @@ int launch_diffusion_vjp(const gem_grid* g, DiffAdjArgs a, cudaStream_t st) {
   long long nblk = (ncs + wpb - 1) / wpb;
   const long long cap = (long long)num_sms() * std::max(best_per_sm, 1);
   if (nblk > cap) nblk = cap;
-  kern<<<(unsigned)nblk, 32 * wpb, smem, st>>>(a);
+  step_launch(kern, (unsigned)nblk, 32 * wpb, smem, st, a);
   GEM_LAUNCHED("k_diffusion_vjp");
   return GEM_OK;
 }
@@ -958,7 +975,7 @@ int gem_work_set_top_temperature(gem_work* w, const double* Ttop, int on_device)
   int name(const gem_grid* g, Fp fluidvars, Ap fluidauxvars, void* stream) {           \
     if (check_grid(g) || !fluidvars || !fluidauxvars) return set_err(GEM_EINVAL, "null argument"); \
     Blocks B = blocks(g, const_cast<double*>(fluidvars), const_cast<double*>(fluidauxvars)); \
-    kern<<<grid_for(g->dev.d.ng, 256), 256, 0, S(stream)>>>(B);                        \
+    step_launch(kern, grid_for(g->dev.d.ng, 256), 256, 0, S(stream), B);               \
     GEM_LAUNCHED(#kern);                                                               \
     return GEM_OK;                                                                     \
   }
@@ -981,7 +998,7 @@ int gem_halo_fluidvars_dev(const gem_grid* g, double* fluidvars, double* fluidau
   if (!g->dev.flagper) return GEM_OK;
   if (g->dev.d.lx3 < 2) return set_err(GEM_EINVAL, "periodic x3 needs lx3 >= 2");
   const long long n = (long long)(g->dev.d.lx1 + 4) * g->dev.d.lx2 * LSP;
-  k_halo_wrap<<<grid_for(n, 128), 128, 0, S(stream)>>>(g->dev, blocks(g, fluidvars, fluidauxvars), 1);
+  step_launch(k_halo_wrap, grid_for(n, 128), 128, 0, S(stream), g->dev, blocks(g, fluidvars, fluidauxvars), 1);
   GEM_LAUNCHED("k_halo_wrap");
   return GEM_OK;
 }
@@ -991,7 +1008,7 @@ int gem_halo_allparams_dev(const gem_grid* g, double* fluidvars, double* fluidau
   if (!g->dev.flagper) return GEM_OK;
   if (g->dev.d.lx3 < 2) return set_err(GEM_EINVAL, "periodic x3 needs lx3 >= 2");
   const long long n = (long long)(g->dev.d.lx1 + 4) * g->dev.d.lx2 * LSP;
-  k_halo_wrap<<<grid_for(n, 128), 128, 0, S(stream)>>>(g->dev, blocks(g, fluidvars, fluidauxvars), 0);
+  step_launch(k_halo_wrap, grid_for(n, 128), 128, 0, S(stream), g->dev, blocks(g, fluidvars, fluidauxvars), 0);
   GEM_LAUNCHED("k_halo_wrap");
   return GEM_OK;
 }
@@ -1001,7 +1018,7 @@ int gem_interface_vels_allspec_dev(const gem_grid* g, const double* fluidvars, g
   if (check_grid(g) || !fluidvars || !w) return set_err(GEM_EINVAL, "null argument");
   if (lsp < 1 || lsp > LSP) return set_err(GEM_EINVAL, "number of interface vels must be in 1..%d", LSP);
   const Dims& d = g->dev.d;
-  k_interface_vels<<<dim3(grid_for(nf1(d) + nf2(d) + nf3(d), 256, 4), lsp), 256, 0, S(stream)>>>(
+  step_launch(k_interface_vels, dim3(grid_for(nf1(d) + nf2(d) + nf3(d), 256, 4), lsp), 256, 0, S(stream), 
       g->dev, blocks(g, const_cast<double*>(fluidvars), nullptr), w->vs1i, w->vs2i, w->vs3i);
   GEM_LAUNCHED("k_interface_vels");
   return GEM_OK;
@@ -1027,11 +1044,11 @@ int gem_clean_param_dev(const gem_grid* g, int iparm, double* fluidvars, void* s
   if (iparm < 1 || iparm > 3) return set_err(GEM_EINVAL, "non-standard parameter selected in clean_params");
   const long long ng = g->dev.d.ng;
   double* param = fluidvars + (iparm == 1 ? 0 : iparm == 2 ? LSP : 4 * LSP) * ng;
-  k_clean_elementwise<<<grid_for(ng, 256), 256, 0, S(stream)>>>(g->dev, param, iparm);
+  step_launch(k_clean_elementwise, grid_for(ng, 256), 256, 0, S(stream), g->dev, param, iparm);
   GEM_LAUNCHED("k_clean_elementwise");
   if (iparm == 2 && g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
     const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * LSP;
-    k_clean_vel_edges<<<grid_for(n, 128), 128, 0, S(stream)>>>(g->dev, param);
+    step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, S(stream), g->dev, param);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
   return GEM_OK;
@@ -1039,11 +1056,11 @@ int gem_clean_param_dev(const gem_grid* g, int iparm, double* fluidvars, void* s
 
 // clean_param(3), (2), (1) in the order the source sub-step ends with
 static int clean_all(const gem_grid* g, double* fluidvars, cudaStream_t st) {
-  k_clean_all<<<grid_for(g->dev.d.ng, 256), 256, 0, st>>>(g->dev, blocks(g, fluidvars, nullptr));
+  step_launch(k_clean_all, grid_for(g->dev.d.ng, 256), 256, 0, st, g->dev, blocks(g, fluidvars, nullptr));
   GEM_LAUNCHED("k_clean_all");
   if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
     const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * LSP;
-    k_clean_vel_edges<<<grid_for(n, 128), 128, 0, st>>>(g->dev, fluidvars + LSP * g->dev.d.ng);
+    step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * g->dev.d.ng);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
   return GEM_OK;
@@ -1069,7 +1086,7 @@ int gem_energy_diffusion_dev(const gem_cfg* cfg, const gem_grid* g, double* flui
   a.fused = 0;
   int rc = launch_diffusion(g, a, S(stream));
   if (rc) return rc;
-  k_diffusion_ghost_floor<<<grid_for(g->dev.d.ng, 256), 256, 0, S(stream)>>>(g->dev, a.B);
+  step_launch(k_diffusion_ghost_floor, grid_for(g->dev.d.ng, 256), 256, 0, S(stream), g->dev, a.B);
   GEM_LAUNCHED("k_diffusion_ghost_floor");
   return GEM_OK;
 }
@@ -1082,7 +1099,7 @@ int gem_dt_calc_dev(const gem_grid* g, double tcfl, const double* fluidvars, gem
   Blocks B = blocks(g, const_cast<double*>(fluidvars), nullptr);
   const unsigned nb = dt_blocks(g->dev.d);
   auto kern = g->dev.unit ? k_dt_calc<true> : k_dt_calc<false>;
-  kern<<<nb, dim3(32, LSP), 0, st>>>(g->dev, B, w->dtpart, w->acc + 30, tcfl, dt_out);
+  step_launch(kern, nb, dim3(32, LSP), 0, st, g->dev, B, w->dtpart, w->acc + 30, tcfl, dt_out);
   GEM_LAUNCHED("k_dt_calc");
   w->timer.record(1, st);
   return GEM_OK;
@@ -1248,11 +1265,11 @@ static int fluid_adv_impl(const gem_cfg* cfg, const gem_grid* g, double* fluidva
   w->timer.record(4, st);
   if ((rc = launch_sweep(g, 2, true, a, LSP, st))) return rc;
   w->timer.record(5, st);
-  k_ghost_epilogue<<<grid_for(ghost_cells(g->dev.d), 256), 256, 0, st>>>(g->dev, B);
+  step_launch(k_ghost_epilogue<false>, grid_for(ghost_cells(g->dev.d), 256), 256, 0, st, g->dev, B);
   GEM_LAUNCHED("k_ghost_epilogue");
   if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
     const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * LSP;
-    k_clean_vel_edges<<<grid_for(n, 128), 128, 0, st>>>(g->dev, fluidvars + LSP * g->dev.d.ng);
+    step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * g->dev.d.ng);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
   if (after_epi) GEM_CUDA(cudaEventRecord(after_epi, st));
@@ -1303,15 +1320,15 @@ static int advection_keepre(const gem_grid* g, double* fluidvars, double* fluida
   if ((rc = launch_sweep(g, 1, true, a, LSP, st))) return rc;
   const dim3 block(32, LSP), grid((d.lx1 + 31) / 32, d.lx3, a.nsB ? sweep_parts(d, 2) : 1);
   if (g->dev.unit)
-    k_sweep_march<2, true, true, 2, true><<<grid, block, 0, st>>>(a);
+    step_launch(k_sweep_march<2, true, true, 2, true>, grid, block, 0, st, a);
   else
-    k_sweep_march<2, false, true, 2, true><<<grid, block, 0, st>>>(a);
+    step_launch(k_sweep_march<2, false, true, 2, true>, grid, block, 0, st, a);
   GEM_LAUNCHED("k_sweep_march");
-  k_ghost_epilogue<true><<<grid_for(ghost_cells(d), 256), 256, 0, st>>>(g->dev, B);
+  step_launch(k_ghost_epilogue<true>, grid_for(ghost_cells(d), 256), 256, 0, st, g->dev, B);
   GEM_LAUNCHED("k_ghost_epilogue");
   if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
     const long long n = (long long)d.lx2 * d.lx3 * LSP;
-    k_clean_vel_edges<<<grid_for(n, 128), 128, 0, st>>>(g->dev, fluidvars + LSP * d.ng);
+    step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * d.ng);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
   return GEM_OK;
@@ -1336,7 +1353,7 @@ static int diffusion_clean_T2rhoe(const gem_cfg* cfg, const gem_grid* g, double*
   a.solver = cfg->diffsolvetype;
   a.fused = 1;
   if ((rc = launch_diffusion(g, a, st))) return rc;
-  k_ghost_T100<<<grid_for(ghost_cells(g->dev.d), 256), 256, 0, st>>>(g->dev, a.B);
+  step_launch(k_ghost_T100, grid_for(ghost_cells(g->dev.d), 256), 256, 0, st, g->dev, a.B);
   GEM_LAUNCHED("k_ghost_T100");
   return GEM_OK;
 }

@@ -44,8 +44,8 @@ int gem_fluid_adv_compression_dev(const gem_cfg* cfg, const gem_grid* g, double*
     // one pass over the interior cells, then the ghost velocities
     const dim3 grid(grid_for(nci(d), 256), LSP);
     const Blocks B = blocks(g, fluidvars, fluidauxvars);
-    if (g->dev.unit) gemk::kc_compress_T<true><<<grid, 256, 0, S(stream)>>>(g->dev, B, Q, dt);
-    else gemk::kc_compress_T<false><<<grid, 256, 0, S(stream)>>>(g->dev, B, Q, dt);
+    if (g->dev.unit) step_launch(gemk::kc_compress_T<true>, grid, 256, 0, S(stream), g->dev, B, Q, dt);
+    else step_launch(gemk::kc_compress_T<false>, grid, 256, 0, S(stream), g->dev, B, Q, dt);
     GEM_LAUNCHED("kc_compress_T");
     GEM_TRY(gem_halo_fluidvars_dev(g, fluidvars, fluidauxvars, stream));
     GEM_TRY(gem_rk2_global_boundary_allspec_dev(g, fluidvars, stream));

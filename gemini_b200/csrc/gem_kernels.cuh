@@ -54,6 +54,15 @@ __constant__ double c_tcoef[LSP - 1] = {(double)0.1019e-12f, (double)0.0747e-12f
                                         (double)0.0754e-12f, (double)0.0701e-12f,
                                         (double)0.1068e-12f, (double)0.3986e-12f};
 
+// First statement of the kernels of a step, which are launched with programmatic stream
+// serialization (step_launch): the launch overlaps the previous kernel's end, and this waits
+// until that kernel has completed and its writes are visible.  No kernel releases the next one
+// early: blocks that wait beside the running ones slowed the large grids (384x192x192 14.5 ->
+// 15.4 ms).  64x8x6 step 95 -> 78 us, 96x32x32 210 -> 191.
+__device__ __forceinline__ void step_entry() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 struct Dims {
   int lx1, lx2, lx3;
   long long s2, s3, ng;
@@ -205,18 +214,21 @@ __device__ __forceinline__ double conv_re(double n, double T, int s) { return md
 // 2. Elementwise conversions over the full ghosted arrays (multifluid.f90:179-233)
 // ======================================================================================
 __global__ void k_v12rhov1(Blocks B) {
+  step_entry();
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < B.ng;
        k += (long long)gridDim.x * blockDim.x)
     for (int s = 0; s < LSP; ++s) B.rv(s)[k] = conv_rv(B.ns(s)[k], B.vs1(s)[k], s);
 }
 
 __global__ void k_T2rhoe(Blocks B) {
+  step_entry();
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < B.ng;
        k += (long long)gridDim.x * blockDim.x)
     for (int s = 0; s < LSP; ++s) B.re(s)[k] = conv_re(B.ns(s)[k], B.Ts(s)[k], s);
 }
 
 __global__ void k_rhoe2T(Blocks B) {
+  step_entry();
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < B.ng;
        k += (long long)gridDim.x * blockDim.x)
     for (int s = 0; s < LSP; ++s) {
@@ -226,6 +238,7 @@ __global__ void k_rhoe2T(Blocks B) {
 }
 
 __global__ void k_rhov12v1(Blocks B) {
+  step_entry();
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < B.ng;
        k += (long long)gridDim.x * blockDim.x) {
     double chrg = 0.0, nsum = 0.0;
@@ -299,6 +312,7 @@ __device__ __forceinline__ void ghost_cell(const Dims& d, long long q, int& i1, 
 
 // param: the 4-D block of ns (1), vs1 (2) or Ts (3), all lsp species
 __global__ void k_clean_elementwise(GridDev G, double* param, int iparm) {
+  step_entry();
   const Dims d = G.d;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < d.ng;
        k += (long long)gridDim.x * blockDim.x) {
@@ -334,6 +348,7 @@ __global__ void k_clean_elementwise(GridDev G, double* param, int iparm) {
 // clean already, so a value is stored only where it changes: 14 doubles a cell read instead
 // of 14 read and 14 written in three passes.
 __global__ void k_clean_all(GridDev G, Blocks B) {
+  step_entry();
   const Dims d = G.d;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < d.ng;
        k += (long long)gridDim.x * blockDim.x) {
@@ -387,6 +402,7 @@ __device__ __forceinline__ void b_clean_vel_edges(const GridDev& G, double* vs1,
 }
 
 __global__ void k_clean_vel_edges(GridDev G, double* vs1) {
+  step_entry();
   b_clean_vel_edges(G, vs1, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
@@ -512,6 +528,7 @@ __device__ __forceinline__ void b_ghost_x1(const GridDev& G, const Blocks& B, co
 
 template <bool CONV>
 __global__ void k_ghost_x1(GridDev G, Blocks B, const double* __restrict__ vs1i, int lsp) {
+  step_entry();
   b_ghost_x1<CONV>(G, B, vs1i, lsp, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
@@ -552,6 +569,7 @@ __device__ __forceinline__ void b_ghost_x2(const GridDev& G, const Blocks& B, in
 
 template <bool CONV>
 __global__ void k_ghost_x2(GridDev G, Blocks B, int lsp) {
+  step_entry();
   b_ghost_x2<CONV>(G, B, lsp, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
@@ -612,12 +630,14 @@ __device__ __forceinline__ void b_ghost_x3(const GridDev& G, const Blocks& B, in
 
 template <bool CONV, bool WRAP>
 __global__ void k_ghost_x3(GridDev G, Blocks B, int lsp) {
+  step_entry();
   b_ghost_x3<CONV, WRAP>(G, B, lsp, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
 
 // Halo wrap only (standalone halo_allparams / halo_fluidvars): rows 1:lx2, all x1.
 __global__ void k_halo_wrap(GridDev G, Blocks B, int with_v23) {
+  step_entry();
   const Dims d = G.d;
   const int n1 = d.lx1 + 4;
   const long long nrow = (long long)n1 * d.lx2;
@@ -648,6 +668,7 @@ __global__ void k_halo_wrap(GridDev G, Blocks B, int with_v23) {
 // One thread per face of the three families (enumerated back to back, 32-bit indices: the
 // per-species face counts stay below 2^31), blockIdx.y the species.
 __global__ void k_interface_vels(GridDev G, Blocks B, double* vs1i, double* vs2i, double* vs3i) {
+  step_entry();
   const Dims d = G.d;
   const int n1 = (int)nf1(d), n2 = (int)nf2(d), n3 = (int)nf3(d);
   const int s = blockIdx.y;
@@ -1317,6 +1338,7 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb, i
 // blockIdx.z: the part of the line
 template <int DIM, bool UNIT, bool FUSED, int PERM = 2, bool KEEPRE = false, bool INV = false>
 __global__ void __launch_bounds__(224, GEM_MARCH_MINB) k_sweep_march(SweepArgs P) {
+  step_entry();
   b_sweep_march<DIM, UNIT, FUSED, PERM, KEEPRE, INV>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x},
                                                      (int)blockIdx.z, (int)gridDim.z);
 }
@@ -1325,6 +1347,7 @@ __global__ void __launch_bounds__(224, GEM_MARCH_MINB) k_sweep_march(SweepArgs P
 // three fields out of place (SweepTri); blockIdx.z: field + 3 * part of the line
 template <int DIM, bool UNIT>
 __global__ void __launch_bounds__(224, 2) k_sweep_tri(SweepTri T) {
+  step_entry();
   const int f = blockIdx.z % 3;
   if (threadIdx.y == LSP - 1 && f < 2) return;
   b_sweep_march<DIM, UNIT, false>(T.field(f, DIM), VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x},
@@ -1525,11 +1548,13 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
 
 template <bool UNIT, bool FUSED, bool OOP = false>
 __global__ void __launch_bounds__(224, OOP ? 2 : 3) k_sweep_x1(SweepArgs P) {
+  step_entry();
   b_sweep_x1<UNIT, FUSED, OOP>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
 template <bool UNIT>
 __global__ void __launch_bounds__(224, 3) k_sweep_tri_x1(SweepTri T) {
+  step_entry();
   const int f = blockIdx.z;
   if (threadIdx.y == LSP - 1 && f < 2) return;
   b_sweep_x1<UNIT, false, true>(T.field(f, 1), VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
@@ -1570,12 +1595,14 @@ __device__ __forceinline__ void b_ghost_epilogue(const GridDev& G, const Blocks&
 
 template <bool KEEPRE = false>
 __global__ void k_ghost_epilogue(GridDev G, Blocks B) {
+  step_entry();
   b_ghost_epilogue<KEEPRE>(G, B, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
 // clean_param(3) and T2rhoe on the ghost shell after a fused diffusion store (which covers
 // the interior cells): every ghost temperature 100, rhoes from the cell's density.
 __global__ void k_ghost_T100(GridDev G, Blocks B) {
+  step_entry();
   const Dims d = G.d;
   const long long ngh = nghost(d);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < ngh; q += (long long)gridDim.x * blockDim.x) {
@@ -2107,6 +2134,7 @@ __device__ __forceinline__ void b_diffusion_lu(const DiffArgs& P, int task, doub
 // plain launch: persistent warps over the warp tasks; scratch slot = the global warp index
 template <bool UNIT, int MINB>
 __global__ void __launch_bounds__(32 * LU_WPB, MINB) k_diffusion_lu(DiffArgs P) {
+  step_entry();
   __shared__ LuTiles tiles[LU_WPB];
   const int warp = threadIdx.x >> 5;
   const int gw = blockIdx.x * LU_WPB + warp;
@@ -2319,6 +2347,7 @@ __device__ __forceinline__ void b_diffusion_col(const DiffArgs& P, int s, int co
 
 template <bool UNIT>
 __global__ void __launch_bounds__(LUC_THREADS, 4) k_diffusion_col(DiffArgs P, int cb) {
+  step_entry();
   extern __shared__ double luc_w[];
   const int ncol = P.G.d.lx2 * P.G.d.lx3;
   const int ng = (ncol + cb - 1) / cb;
@@ -2337,6 +2366,7 @@ __global__ void __launch_bounds__(LUC_THREADS, 4) k_diffusion_col(DiffArgs P, in
 
 // standalone energy_diffusion: max(T,100) on the ghost cells other than the x1 BC layers
 __global__ void k_diffusion_ghost_floor(GridDev G, Blocks B) {
+  step_entry();
   const Dims d = G.d;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < d.ng;
        k += (long long)gridDim.x * blockDim.x) {
@@ -2431,6 +2461,7 @@ __device__ __forceinline__ void lam_deriv(int s, double T, double nv, double n1,
 
 template <bool UNIT>
 __global__ void __launch_bounds__(128) k_diffusion_vjp(DiffAdjArgs P) {
+  step_entry();
   extern __shared__ double smem[];
   const GridDev& G = P.G;
   const Dims d = G.d;
@@ -2896,6 +2927,7 @@ __device__ __forceinline__ SlopeBr slope_br(const Line1D& L, int k, double fm, d
 
 template <int DIM, bool UNIT>
 __global__ void __launch_bounds__(256, 3) k_sweep_vjp_march(SweepVjpArgs P, SweepVjpFields FS, int nseg) {
+  step_entry();
   const GridDev& G = P.G;
   const Dims d = G.d;
   const int lx = (DIM == 2) ? d.lx2 : d.lx3;
@@ -3028,6 +3060,7 @@ __global__ void __launch_bounds__(256, 3) k_sweep_vjp_march(SweepVjpArgs P, Swee
 // chunk and the previous one.  Face-velocity cotangents go to the field's own vbar slice.
 template <bool UNIT>
 __global__ void __launch_bounds__(256, 3) k_sweep_vjp_x1(SweepVjpArgs P, SweepVjpFields FS) {
+  step_entry();
   const GridDev& G = P.G;
   const Dims d = G.d;
   const int lx = d.lx1;
@@ -3295,6 +3328,7 @@ template <bool UNIT>
 __global__ void __launch_bounds__(32 * LSP, GEM_DT_MINB) k_dt_calc(GridDev G, Blocks B, double* part,
                                                                    unsigned long long* count, double tcfl,
                                                                    double* dt_out) {
+  step_entry();
   b_dt_reduce<UNIT, 0>(G, B, nullptr, nullptr, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x}, part);
   __shared__ bool last;
   __shared__ double inv[LSP];

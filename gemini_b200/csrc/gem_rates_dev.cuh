@@ -14,6 +14,7 @@ struct RateIn {  // interior neutral inputs
 
 __global__ void kr_continuity(gemr::View v, RateIn in, const double* __restrict__ fv, double* __restrict__ Pr,
                               double* __restrict__ Lo) {
+  step_entry();
   const long long n = gemr::ncell(v);
   const double *ns = fv, *vs1 = fv + LSP * v.ng, *vs2 = fv + 2 * LSP * v.ng, *vs3 = fv + 3 * LSP * v.ng,
                *Ts = fv + 4 * LSP * v.ng;
@@ -138,6 +139,7 @@ __device__ __forceinline__ bool load_cells(const gemr::View& v, const double* __
 // fast quotients and the shared cell table, 2.83 ms.
 __global__ void __launch_bounds__(kRateThreads, 5) kr_energy(gemr::View v, RateIn in, const double* __restrict__ fv,
                                                           double* __restrict__ Pr, double* __restrict__ Lo) {
+  step_entry();
   __shared__ PairTab tab;
   __shared__ CellTab cells;
   const int isp = threadIdx.x / kRateCells, lane = threadIdx.x % kRateCells;
@@ -188,6 +190,7 @@ __global__ void __launch_bounds__(kRateThreads, 5) kr_momentum(gemr::View v, Rat
                                                             const double* __restrict__ alt,
                                                             const double* __restrict__ g1, double* __restrict__ Pr,
                                                             double* __restrict__ Lo) {
+  step_entry();
   __shared__ PairTab tab;
   __shared__ CellTab cells;
   __shared__ double s_epol[kRateCells];
@@ -283,7 +286,7 @@ int gem_srcs_continuity_dev(const gem_grid* g, const double* nn, const double* v
     return set_err(GEM_EINVAL, "null argument");
   const gemr::View v = gemk::rate_view(g);
   const long long n = gemr::ncell(v);
-  gemk::kr_continuity<<<grid_for(n, 128), 128, 0, S(stream)>>>(v, gemk::RateIn{nn, vn1, vn2, vn3, Tn}, fluidvars,
+  step_launch(gemk::kr_continuity, grid_for(n, 128), 128, 0, S(stream), v, gemk::RateIn{nn, vn1, vn2, vn3, Tn}, fluidvars,
                                                                   Pr, Lo);
   GEM_LAUNCHED("kr_continuity");
   return GEM_OK;
@@ -295,7 +298,7 @@ int gem_srcs_energy_dev(const gem_grid* g, const double* nn, const double* vn1, 
     return set_err(GEM_EINVAL, "null argument");
   const gemr::View v = gemk::rate_view(g);
   const long long nb = (gemr::ncell(v) + gemk::kRateCells - 1) / gemk::kRateCells;
-  gemk::kr_energy<<<(unsigned)nb, gemk::kRateThreads, 0, S(stream)>>>(v, gemk::RateIn{nn, vn1, vn2, vn3, Tn}, fluidvars, Pr,
+  step_launch(gemk::kr_energy, (unsigned)nb, gemk::kRateThreads, 0, S(stream), v, gemk::RateIn{nn, vn1, vn2, vn3, Tn}, fluidvars, Pr,
                                                               Lo);
   GEM_LAUNCHED("kr_energy");
   return GEM_OK;
@@ -309,7 +312,7 @@ int gem_srcs_momentum_dev(const gem_grid* g, const double* nn, const double* vn1
   if (g->dev.d.lx1 < 2) return set_err(GEM_EINVAL, "the x1 gradients need lx1 >= 2");
   const gemr::View v = gemk::rate_view(g);
   const long long nb = (gemr::ncell(v) + gemk::kRateCells - 1) / gemk::kRateCells;
-  gemk::kr_momentum<<<(unsigned)nb, gemk::kRateThreads, 0, S(stream)>>>(v, gemk::RateIn{nn, vn1, nullptr, nullptr, Tn},
+  step_launch(gemk::kr_momentum, (unsigned)nb, gemk::kRateThreads, 0, S(stream), v, gemk::RateIn{nn, vn1, nullptr, nullptr, Tn},
                                                                 fluidvars, electrovars, Q, alt, g1, Pr, Lo);
   GEM_LAUNCHED("kr_momentum");
   return GEM_OK;

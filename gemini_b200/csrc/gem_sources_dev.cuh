@@ -9,6 +9,7 @@ namespace gemk {
 __global__ void ks_mass(gems::View v, double* __restrict__ Pr, const double* __restrict__ Lo,
                         const double* __restrict__ Prprecip, double* __restrict__ ns,
                         const double* __restrict__ dtp) {
+  step_entry();
   const double dt = *dtp;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < v.ng; k += (long long)gridDim.x * blockDim.x)
     gems::mass_cell(v, k, dt, Pr, Lo, Prprecip, ns);
@@ -16,6 +17,7 @@ __global__ void ks_mass(gems::View v, double* __restrict__ Pr, const double* __r
 __global__ void ks_momentum(gems::View v, const double* __restrict__ Pr, const double* __restrict__ Lo,
                             const double* __restrict__ ns, double* __restrict__ rhovs1, double* __restrict__ vs1,
                             const double* __restrict__ dtp) {
+  step_entry();
   const double dt = *dtp;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < v.ng; k += (long long)gridDim.x * blockDim.x)
     gems::momentum_cell(v, k, dt, Pr, Lo, ns, rhovs1, vs1);
@@ -23,6 +25,7 @@ __global__ void ks_momentum(gems::View v, const double* __restrict__ Pr, const d
 __global__ void ks_energy(gems::View v, double* __restrict__ Pr, const double* __restrict__ Lo,
                           const double* __restrict__ Qeprecip, double* __restrict__ rhoes, double* __restrict__ Ts,
                           const double* __restrict__ ns, const double* __restrict__ dtp) {
+  step_entry();
   const double dt = *dtp;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < v.ng; k += (long long)gridDim.x * blockDim.x)
     gems::energy_cell(v, k, dt, Pr, Lo, Qeprecip, rhoes, Ts, ns);
@@ -55,7 +58,7 @@ int gem_mass_source_loss_solve_dev(const gem_grid* g, const double* dt, double* 
                                    const double* Prprecip, double* fluidvars, void* stream) {
   if (check_grid(g) || !dt || !Pr || !Lo || !Prprecip || !fluidvars) return set_err(GEM_EINVAL, "null argument");
   const gems::View v = gemk::src_view(g);
-  gemk::ks_mass<<<grid_for(v.ng, 256), 256, 0, S(stream)>>>(v, Pr, Lo, Prprecip, fluidvars, dt);
+  step_launch(gemk::ks_mass, grid_for(v.ng, 256), 256, 0, S(stream), v, Pr, Lo, Prprecip, fluidvars, dt);
   GEM_LAUNCHED("ks_mass");
   return GEM_OK;
 }
@@ -64,7 +67,7 @@ int gem_momentum_source_loss_solve_dev(const gem_grid* g, const double* dt, cons
                                        double* fluidvars, double* fluidauxvars, void* stream) {
   if (check_grid(g) || !dt || !Pr || !Lo || !fluidvars || !fluidauxvars) return set_err(GEM_EINVAL, "null argument");
   const gems::View v = gemk::src_view(g);
-  gemk::ks_momentum<<<grid_for(v.ng, 256), 256, 0, S(stream)>>>(v, Pr, Lo, fluidvars, fluidauxvars,
+  step_launch(gemk::ks_momentum, grid_for(v.ng, 256), 256, 0, S(stream), v, Pr, Lo, fluidvars, fluidauxvars,
                                                                  fluidvars + LSP * v.ng, dt);
   GEM_LAUNCHED("ks_momentum");
   return GEM_OK;
@@ -75,7 +78,7 @@ int gem_energy_source_loss_solve_dev(const gem_grid* g, const double* dt, double
   if (check_grid(g) || !dt || !Pr || !Lo || !Qeprecip || !fluidvars || !fluidauxvars)
     return set_err(GEM_EINVAL, "null argument");
   const gems::View v = gemk::src_view(g);
-  gemk::ks_energy<<<grid_for(v.ng, 256), 256, 0, S(stream)>>>(v, Pr, Lo, Qeprecip, fluidauxvars + LSP * v.ng,
+  step_launch(gemk::ks_energy, grid_for(v.ng, 256), 256, 0, S(stream), v, Pr, Lo, Qeprecip, fluidauxvars + LSP * v.ng,
                                                                fluidvars + 4 * LSP * v.ng, fluidvars, dt);
   GEM_LAUNCHED("ks_energy");
   return GEM_OK;
