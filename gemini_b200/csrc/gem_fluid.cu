@@ -131,8 +131,8 @@ struct gem_work {
   int lx1, lx2, lx3;
   double *vs1i, *vs2i, *vs3i, *nn, *Tn, *dt;
   double* Ttop;             // per-column exospheric temperature (lx2*lx3), or null for Teinf
-  double* lu;               // band-solve scratch of k_diffusion_lu (lu_slots() slots of lx1 rows)
-  double* sweep;            // out-of-place blocks of the fused sweeps on small grids
+  double* lu;               // the step's scratch (work_scratch): the diffusion's
+  double* sweep;            // and, behind it, the out-of-place blocks of the cut sweeps
   // the reference work object's sub-step contents for the host-memory *_C routines, allocated
   // on first use: the neutral state and ionization rates (gem_work_set_sources) and the
   // artificial viscosity Q, production and loss rates Pr, Lo
@@ -193,18 +193,16 @@ int sweep_parts(const Dims& d, int dim) {
   return (int)std::max<long long>(1, std::min<long long>(2LL * num_sms() / blocks, lx / 4));
 }
 
+int work_scratch(gem_work* w, const gem_grid* g);
+
 // The out-of-place blocks of the fused sweeps where a line is cut (else null): densities,
-// momentum and energy densities of all species, allocated by the first step.
+// momentum and energy densities of all species.
+bool sweeps_cut(const Dims& d) { return sweep_parts(d, 2) > 1 || sweep_parts(d, 3) > 1; }
 int work_sweeps(gem_work* w, const gem_grid* g, SweepArgs& a) {
   const Dims& d = g->dev.d;
-  if (sweep_parts(d, 2) == 1 && sweep_parts(d, 3) == 1) return GEM_OK;
-  if (!w->sweep) {
-    const size_t bytes = sizeof(double) * 3 * LSP * d.ng;
-    if (cudaMalloc(&w->sweep, bytes) != cudaSuccess) {
-      w->sweep = nullptr;
-      return set_err(GEM_ENOMEM, "cudaMalloc of %zu bytes for the sweeps' scratch failed", bytes);
-    }
-  }
+  if (!sweeps_cut(d)) return GEM_OK;
+  const int rc = work_scratch(w, g);
+  if (rc) return rc;
   a.nsB = w->sweep;
   a.rvB = a.nsB + LSP * d.ng;
   a.reB = a.rvB + LSP * d.ng;
@@ -329,20 +327,6 @@ long long lu_tasks(const Dims& d) {
 // scratch slots a grid's launches use: one per resident warp, no more than it has tasks
 long long lu_slots_for(const Dims& d) { return std::min(lu_slots(), lu_tasks(d)); }
 
-// The work object's band-solve scratch, allocated by the first diffusion launch that uses
-// the work object (the batched step uses its own; a work object only ever batched needs none).
-int work_lu(gem_work* w, const gem_grid* g, double** out) {
-  if (!w->lu) {
-    const size_t bytes = sizeof(double) * lu_slots_for(g->dev.d) * lu_slot_doubles(g->dev.d.lx1);
-    if (cudaMalloc(&w->lu, bytes) != cudaSuccess) {
-      w->lu = nullptr;
-      return set_err(GEM_ENOMEM, "cudaMalloc of %zu bytes for the diffusion's band-solve scratch failed", bytes);
-    }
-  }
-  *out = w->lu;
-  return GEM_OK;
-}
-
 // Columns per block of k_diffusion_col, 0 where k_diffusion_lu runs instead.
 // k_diffusion_lu takes about 2 us per x1 row however few columns there are (one thread's
 // chain through four passes) and slows down only beyond 12 warps per SM.  k_diffusion_col
@@ -365,6 +349,29 @@ int luc_columns(const Dims& d) {
   const long long want = std::max<long long>(1, (std::min(per_sm, fit) + 3) / 4);
   const long long most = std::max<long long>(1, (long long)((SM_BYTES / 4 - BLOCK_OVERHEAD) / luc_bytes(d.lx1)));
   return (int)std::min<long long>(32, std::min(want, most));
+}
+
+// The work object's scratch, one allocation by the first launch that needs any of it (two
+// would cost a small grid's first step 0.3 ms more): the diffusion's, the factors of every
+// column for k_diffusion_col or a slot per resident warp for k_diffusion_lu, then the cut
+// sweeps' blocks.  The batched step has its own; a work object only ever batched needs none.
+int work_scratch(gem_work* w, const gem_grid* g) {
+  if (w->lu) return GEM_OK;
+  const Dims& d = g->dev.d;
+  const long long lu = luc_columns(d) > 0 ? 3LL * LSP * nci(d) : lu_slots_for(d) * lu_slot_doubles(d.lx1);
+  const size_t bytes = sizeof(double) * (size_t)(lu + (sweeps_cut(d) ? 3LL * LSP * d.ng : 0));
+  if (cudaMalloc(&w->lu, bytes) != cudaSuccess) {
+    w->lu = nullptr;
+    return set_err(GEM_ENOMEM, "cudaMalloc of %zu bytes for the step's scratch failed", bytes);
+  }
+  w->sweep = w->lu + lu;
+  return GEM_OK;
+}
+
+int work_lu(gem_work* w, const gem_grid* g, double** out) {
+  const int rc = work_scratch(w, g);
+  *out = w->lu;
+  return rc;
 }
 
 int launch_diffusion_lu(const gem_grid* g, DiffArgs a, cudaStream_t st) {
@@ -544,7 +551,9 @@ int gem_grid_create(const gem_grid_desc* desc, gem_grid** out) {
                n3 = (size_t)lx1 * lx2 * (lx3 + 1);
   // the sweeps' shared range tests assume narrower reciprocals; others take the slow path
   auto narrow = [&](double y) {
-    if (!(std::fabs(y) >= std::ldexp(1.0, -200) && std::fabs(y) <= std::ldexp(1.0, 200))) G.wide = 1;
+    unsigned long long u;
+    std::memcpy(&u, &y, 8);
+    if (((unsigned)(u >> 32) & 0x7fffffffu) - (823u << 20) >= (400u << 20)) G.wide = 1;
   };
   G.wide = 0;
   const double* need[] = {desc->dx1, desc->dx1i, desc->dx2, desc->dx2i, desc->dx3, desc->dx3i,
@@ -821,7 +830,7 @@ int gem_work_destroy(gem_work* w) {
   for (cudaEvent_t e : w->ev)
     if (e) cudaEventDestroy(e);
   if (w->cs) cudaStreamDestroy(w->cs);
-  void* ps[] = {w->vs1i, w->vs2i, w->vs3i, w->nn, w->Tn, w->dt, w->acc, w->dtpart, w->F, w->A, w->E, w->Ttop, w->lu, w->sweep, w->sub};
+  void* ps[] = {w->vs1i, w->vs2i, w->vs3i, w->nn, w->Tn, w->dt, w->acc, w->dtpart, w->F, w->A, w->E, w->Ttop, w->lu, w->sub};
   for (void* p : ps)
     if (p) cudaFree(p);
   delete w;
@@ -904,10 +913,7 @@ int gem_work_prepare(gem_work* w, const gem_grid* g) {
   if (!w || check_grid(g)) return set_err(GEM_EINVAL, "null argument");
   if (w->lx1 != g->dev.d.lx1 || w->lx2 != g->dev.d.lx2 || w->lx3 != g->dev.d.lx3)
     return set_err(GEM_EINVAL, "work object and grid sizes differ");
-  double* p = nullptr;
-  SweepArgs a;
-  const int rc = work_lu(w, g, &p);
-  return rc ? rc : work_sweeps(w, g, a);
+  return work_scratch(w, g);
 }
 
 int gem_work_substep_buffers(gem_work* w, const gem_source_inputs** src, double** Q, double** Pr, double** Lo) {
