@@ -43,10 +43,11 @@ __global__ void kb_set_dt(const InstDev* inst, const double* dt_in, int ninst) {
 }
 
 // the time step of each instance from its maxima (k_dt_calc's formula)
-__global__ void kb_dt_finalize(const InstDev* inst, int ninst) {
+__global__ void kb_dt_finalize(const InstDev* inst, int ninst, int unit) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ninst) return;
   const InstDev& I = inst[i];
+  if ((I.sw.G.unit != 0) != (unit != 0)) return;
   double m = 0.0;
   for (int q = 0; q < 3 * LSP; ++q) {
     const double gr = fmax_f(__longlong_as_double((long long)I.acc[q]), 1e-10);
@@ -183,7 +184,13 @@ struct gem_batch {
   cudaGraph_t graph_fixed = nullptr;  // the step with prescribed time steps
   cudaGraphExec_t exec_fixed = nullptr;
   double* d_dt_in = nullptr;  // per-instance prescribed dt (device)
-  double* d_lu = nullptr;     // band-solve scratch shared by the instances' diffusion items
+  // band-solve scratch of the instances' diffusion items, one per metric variant that has any
+  double *d_lu[2] = {nullptr, nullptr}, *lu_base[2] = {nullptr, nullptr};
+  // the two variants' instances share nothing, so their launches run as two chains: where one
+  // chain's phase thins out, the other's blocks fill the device (eight instances 14.7 -> 13.15 ms)
+  bool variant[2] = {false, false}, two = false;
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   long long lu_slot = 0;      // doubles per scratch slot (the longest column's)
   int use_graph = 1;
 };
@@ -261,17 +268,15 @@ int batch_build_lists(gem_batch* b) {
         const gem_grid* g = b->grids[i];
         const Dims& d = g->dev.d;
         const bool unit = g->dev.unit != 0;
-        const bool variant = (k == BK_DT || k == BK_SW3 || k == BK_SW1 || k == BK_SW2 || k == BK_DIFF);
-        if (variant && unit != (u == 1)) continue;
-        if (!variant && u == 0) continue;  // unsplit phases: once
+        if (unit != (u == 1)) continue;
         const int gx13 = (d.lx1 + 31) / 32;
         switch (k) {
           case BK_DT:
             add_items(launch_for(k, u), i, std::min<long long>((long long)d.lx2 * d.lx3, (long long)num_sms() * 8));
             break;
-          case BK_GX1: add_items(launch_for(k, 0), i, grid_for(ghost_x1_items(d, g->dev.flagper, LSP, true), 128)); break;
-          case BK_GX2: add_items(launch_for(k, 0), i, grid_for((long long)(d.lx1 + 4) * (d.lx3 + 4) * LSP, 128)); break;
-          case BK_GX3: add_items(launch_for(k, 0), i, grid_for((long long)(d.lx1 + 4) * (d.lx2 + 4) * LSP, 128)); break;
+          case BK_GX1: add_items(launch_for(k, u), i, grid_for(ghost_x1_items(d, g->dev.flagper, LSP, true), 128)); break;
+          case BK_GX2: add_items(launch_for(k, u), i, grid_for((long long)(d.lx1 + 4) * (d.lx3 + 4) * LSP, 128)); break;
+          case BK_GX3: add_items(launch_for(k, u), i, grid_for((long long)(d.lx1 + 4) * (d.lx2 + 4) * LSP, 128)); break;
           case BK_SW3: {
             BatchLaunch& L = launch_for(k, u);
             L.inv = L.inv && g->dev.c3 == 0;
@@ -281,10 +286,10 @@ int batch_build_lists(gem_batch* b) {
           }
           case BK_SW1: add_items(launch_for(k, u), i, d.lx2, d.lx3); break;
           case BK_SW2: add_items(launch_for(k, u), i, gx13, d.lx3); break;
-          case BK_EPI: add_items(launch_for(k, 0), i, grid_for(ghost_cells(d), 256)); break;
+          case BK_EPI: add_items(launch_for(k, u), i, grid_for(ghost_cells(d), 256)); break;
           case BK_CVE:
             if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1))
-              add_items(launch_for(k, 0), i, grid_for((long long)d.lx2 * d.lx3 * LSP, 128));
+              add_items(launch_for(k, u), i, grid_for((long long)d.lx2 * d.lx3 * LSP, 128));
             break;
           case BK_DIFF: {
             const long long ntask = (((long long)d.lx2 * d.lx3 + 31) / 32) * LSP;
@@ -316,20 +321,17 @@ void batch_drop_graph(gem_batch* b) {
   b->graph_fixed = nullptr;
 }
 
-// fixed_dt: the instances' dt slots are loaded from d_dt_in instead of dt_calc
-int batch_enqueue(gem_batch* b, cudaStream_t st, bool fixed_dt = false) {
+// the phases of one metric variant's instances, in order
+int batch_chain(gem_batch* b, int unit, cudaStream_t st, bool fixed_dt) {
   const InstDev* I = b->d_inst;
-  if (fixed_dt)
-    kb_set_dt<<<(b->n + 63) / 64, 64, 0, st>>>(I, b->d_dt_in, b->n);
-  else
-    kb_zero_acc<<<b->n, 32, 0, st>>>(I, b->n);
   bool finalized = fixed_dt;
   for (const auto& L : b->launches) {
+    if (L.unit != unit) continue;
     const int n = (int)L.items.size();
     const bool u = L.unit != 0;
     if (fixed_dt && L.kernel == BK_DT) continue;
     if (L.kernel != BK_DT && !finalized) {
-      kb_dt_finalize<<<(b->n + 63) / 64, 64, 0, st>>>(I, b->n);
+      kb_dt_finalize<<<(b->n + 63) / 64, 64, 0, st>>>(I, b->n, unit);
       finalized = true;
     }
     switch (L.kernel) {
@@ -354,13 +356,35 @@ int batch_enqueue(gem_batch* b, cudaStream_t st, bool fixed_dt = false) {
       case BK_EPI: kb_ghost_epilogue<<<L.grid, 256, 0, st>>>(I, L.d_items, n); break;
       case BK_CVE: kb_clean_vel_edges<<<L.grid, 128, 0, st>>>(I, L.d_items, n); break;
       case BK_DIFF:
-        if (u) kb_diffusion_lu<true><<<L.grid, 32 * LU_WPB, 0, st>>>(I, L.d_items, n, b->d_lu, b->lu_slot);
-        else kb_diffusion_lu<false><<<L.grid, 32 * LU_WPB, 0, st>>>(I, L.d_items, n, b->d_lu, b->lu_slot);
+        if (u) kb_diffusion_lu<true><<<L.grid, 32 * LU_WPB, 0, st>>>(I, L.d_items, n, b->d_lu[L.unit], b->lu_slot);
+        else kb_diffusion_lu<false><<<L.grid, 32 * LU_WPB, 0, st>>>(I, L.d_items, n, b->d_lu[L.unit], b->lu_slot);
         break;
     }
   }
   GEM_LAUNCHED("batched step");
   return GEM_OK;
+}
+
+// fixed_dt: the instances' dt slots are loaded from d_dt_in instead of dt_calc
+int batch_enqueue(gem_batch* b, cudaStream_t st, bool fixed_dt = false) {
+  const InstDev* I = b->d_inst;
+  if (fixed_dt)
+    kb_set_dt<<<(b->n + 63) / 64, 64, 0, st>>>(I, b->d_dt_in, b->n);
+  else
+    kb_zero_acc<<<b->n, 32, 0, st>>>(I, b->n);
+  if (!b->two) {
+    for (int u = 1; u >= 0; --u) {
+      const int rc = b->variant[u] ? batch_chain(b, u, st, fixed_dt) : GEM_OK;
+      if (rc) return rc;
+    }
+    return GEM_OK;
+  }
+  GEM_CUDA(cudaEventRecord(b->fork, st));
+  GEM_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
+  const int rc0 = batch_chain(b, 0, b->side, fixed_dt), rc1 = batch_chain(b, 1, st, fixed_dt);
+  GEM_CUDA(cudaEventRecord(b->join, b->side));
+  GEM_CUDA(cudaStreamWaitEvent(st, b->join, 0));
+  return rc0 ? rc0 : rc1;
 }
 
 }  // namespace
@@ -380,9 +404,18 @@ int gem_batch_create(int n, const gem_grid* const* grids, gem_work* const* works
   for (int i = 0; i < n; ++i)
     if (grids[i]) lx1_max = std::max(lx1_max, grids[i]->dev.d.lx1);
   b->lu_slot = lu_slot_doubles(lx1_max);
-  if (cudaMalloc(&b->d_lu, sizeof(double) * lu_slots() * b->lu_slot) != cudaSuccess) {
+  for (int i = 0; i < n; ++i)
+    if (grids[i]) b->variant[grids[i]->dev.unit ? 1 : 0] = true;
+  const size_t lu_bytes = sizeof(double) * lu_slots() * b->lu_slot;
+  if (cudaMalloc(&b->lu_base[0], lu_bytes) != cudaSuccess) {
     delete b;
     return set_err(GEM_ENOMEM, "cudaMalloc of the batch's band-solve scratch failed");
+  }
+  b->d_lu[0] = b->d_lu[1] = b->lu_base[0];
+  if (b->variant[0] && b->variant[1]) {  // two chains need a scratch each; without room, one chain
+    b->two = cudaMalloc(&b->lu_base[1], lu_bytes) == cudaSuccess;
+    if (b->two) b->d_lu[1] = b->lu_base[1];
+    else cudaGetLastError();
   }
   for (int i = 0; i < n; ++i) {
     const gem_grid* g = grids[i];
@@ -422,7 +455,7 @@ int gem_batch_create(int n, const gem_grid* const* grids, gem_work* const* works
     I.df.dtp = w->dt;
     I.df.Teinf = cfgs[i].Teinf;
     I.df.Ttop = w->Ttop;
-    I.df.lu = b->d_lu;
+    I.df.lu = b->d_lu[I.sw.G.unit ? 1 : 0];
     I.df.lu_slot = b->lu_slot;
     I.df.x3fast = (!g->dev.unit && g->dev.c3 == 0) ? 1 : 0;
     I.df.solver = cfgs[i].diffsolvetype;
@@ -440,7 +473,10 @@ int gem_batch_create(int n, const gem_grid* const* grids, gem_work* const* works
   if (cudaMemcpy(b->d_inst, h.data(), sizeof(InstDev) * n, cudaMemcpyHostToDevice) != cudaSuccess)
     rc = set_err(GEM_ECUDA, "copy of the batch instance table failed");
   if (rc == GEM_OK) rc = batch_build_lists(b);
-  if (rc == GEM_OK && cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking) != cudaSuccess)
+  if (rc == GEM_OK && (cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking) != cudaSuccess ||
+                       cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
+                       cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
+                       cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess))
     rc = set_err(GEM_ECUDA, "cudaStreamCreate failed");
   if (rc != GEM_OK) {
     gem_batch_destroy(b);
@@ -457,7 +493,11 @@ int gem_batch_destroy(gem_batch* b) {
     if (L.d_items) cudaFree(L.d_items);
   if (b->d_inst) cudaFree(b->d_inst);
   if (b->d_dt_in) cudaFree(b->d_dt_in);
-  if (b->d_lu) cudaFree(b->d_lu);
+  for (double* p : b->lu_base)
+    if (p) cudaFree(p);
+  if (b->fork) cudaEventDestroy(b->fork);
+  if (b->join) cudaEventDestroy(b->join);
+  if (b->side) cudaStreamDestroy(b->side);
   if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
   delete b;
   return GEM_OK;
@@ -543,7 +583,7 @@ int gem_batch_info(const gem_batch* b, int* launches_per_step, long long* items_
   if (!b) return set_err(GEM_EINVAL, "null batch");
   long long it = 0;
   for (const auto& L : b->launches) it += (long long)L.items.size();
-  if (launches_per_step) *launches_per_step = (int)b->launches.size() + 2;  // + zero, dt finalize
+  if (launches_per_step) *launches_per_step = (int)b->launches.size() + 1 + (b->variant[0] ? 1 : 0) + (b->variant[1] ? 1 : 0);  // + zero, dt finalize
   if (items_per_step) *items_per_step = it;
   return GEM_OK;
 }
