@@ -3,8 +3,8 @@
 The reference runs one simulation per MPI job; here n independent grids of uneven sizes
 (Cartesian and dipole mixed) share the GPU.  One ``Batch.step()`` equals, for every
 instance, ``dt_calc(tcfl)`` followed by ``fluid_adv`` on that instance, bit for bit: each
-phase is one persistent launch over an (instance, block) work list, and the whole step is
-replayed from a captured CUDA graph (``gem_batch_*`` in include/gem_fluid.h).
+phase is one launch per metric variant over an (instance, block) work list, and the whole
+step is replayed from a captured CUDA graph (``gem_batch_*`` in include/gem_fluid.h).
 
     insts = [(DeviceGrid(g), DeviceState.from_host(dg, st), FluidCfg(st.Teinf)), ...]
     b = Batch(insts)

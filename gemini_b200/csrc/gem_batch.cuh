@@ -1,11 +1,12 @@
 // Batched fluid advance: many independent grids of uneven sizes advanced together.
 //
 // Each phase of the step (dt reduce, dt finalize, the three ghost-fill passes, the x3, x1
-// and x2 sweeps, the ghost epilogue, the null-edge velocity fix and the diffusion) is ONE
-// persistent launch over a work list of (instance, block) items, ordered largest instance
-// first; the block bodies are the plain kernels' bodies (gem_kernels.cuh, b_*), so every
+// and x2 sweeps, the ghost epilogue, the null-edge velocity fix and the diffusion) is one
+// launch per metric variant (unit / tabulated) over a work list of (instance, block) items,
+// ordered largest instance first; the block bodies are the plain kernels' bodies (gem_kernels.cuh, b_*), so every
 // instance computes exactly what gem_dt_calc_dev + gem_fluid_adv_dev compute for it.  The
-// eleven launches of a step are captured once into a CUDA graph and replayed.
+// launches of a step are captured once into a CUDA graph, the two variants as parallel chains
+// (they share nothing), and replayed.
 //
 // Included by gem_fluid.cu (one translation unit with the plain path).
 

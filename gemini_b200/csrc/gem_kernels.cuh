@@ -1,16 +1,14 @@
 // Device code of the B200 fluid-advance library: the MC-limited advection sweeps, the
 // ghost fill that replaces the MPI halo, the state conversions / clean_param epilogues, the
-// warp-parallel TRBDF2 field-aligned diffusion and the CFL reduction.
+// TRBDF2 field-aligned diffusion and the CFL reduction.
 //
 // Layout: the reference's Fortran blocks (x1 fastest, 2 ghosts per side, species slowest),
 // so a Fortran or C caller's cudaMalloc'd blocks are used in place.
 //
-// Arithmetic: the advection, ghost fill, conversions and clean-up reproduce the reference's
-// operation order exactly (compiled with -fmad=false; IEEE division and sqrt), so for
-// identical inputs they are bit-identical to the Fortran routines they restate.  The
-// diffusion assembles the same coefficients with reordered divisions and solves the
-// tridiagonal systems without pivoting; its results agree with an extended-precision
-// solution of the reference's discrete equations to ~1e-13 relative.
+// Arithmetic: every kernel of the step reproduces the reference's operation order exactly
+// (compiled with -fmad=false; IEEE division and sqrt), the diffusion's band solve in LAPACK's
+// order with its row interchanges (gem_diffusion_lu.cuh), so for identical inputs they are
+// bit-identical to the Fortran routines they restate.
 #pragma once
 
 #include <cuda_runtime.h>

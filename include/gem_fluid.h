@@ -69,13 +69,13 @@ int gem_grid_create(const gem_grid_desc* desc, gem_grid** out);
 int gem_grid_destroy(gem_grid* g);
 int gem_grid_dims(const gem_grid* g, int* lx1, int* lx2, int* lx3);
 /* The work object holds the per-grid state of the step (interface velocities, neutral inputs,
- * dt, reductions).  The diffusion's band-solve scratch (one slot of lx1 x 8 x 32 doubles per
- * resident warp, at most ~1 GB for 384-row columns) is allocated by the first
- * gem_energy_diffusion_dev / gem_fluid_adv_dev call that uses the work object: make that
- * first call before capturing these calls in a CUDA graph.  Work objects that only take part
- * in a gem_batch never allocate it (the batch has its own). */
+ * dt, reductions).  The step's scratch (for the diffusion a slot of lx1 + 4 rows per resident
+ * warp, 0.5 GB for 384-row columns; on grids with few lines also blocks for the sweeps) is
+ * allocated by the first gem_energy_diffusion_dev / gem_fluid_adv_dev call that uses the work
+ * object: make that first call before capturing these calls in a CUDA graph.  Work objects
+ * that only take part in a gem_batch never allocate it (the batch has its own). */
 int gem_work_create(const gem_grid* g, gem_work** out);
-/* allocate the work object's diffusion scratch now (before measuring free memory or capturing) */
+/* allocate the work object's scratch now (before measuring free memory or capturing) */
 int gem_work_prepare(gem_work* w, const gem_grid* g);
 int gem_work_destroy(gem_work* w);
 /* copy neutral inputs (host pointers; nn (lx1,lx2,lx3,3), Tn (lx1,lx2,lx3)) */
