@@ -1053,7 +1053,7 @@ int gem_clean_param_dev(const gem_grid* g, int iparm, double* fluidvars, void* s
   step_launch(k_clean_elementwise, grid_for(ng, 256), 256, 0, S(stream), g->dev, param, iparm);
   GEM_LAUNCHED("k_clean_elementwise");
   if (iparm == 2 && g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
-    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * LSP;
+    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * 32;
     step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, S(stream), g->dev, param);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
@@ -1065,7 +1065,7 @@ static int clean_all(const gem_grid* g, double* fluidvars, cudaStream_t st) {
   step_launch(k_clean_all, grid_for(g->dev.d.ng, 256), 256, 0, st, g->dev, blocks(g, fluidvars, nullptr));
   GEM_LAUNCHED("k_clean_all");
   if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
-    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * LSP;
+    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * 32;
     step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * g->dev.d.ng);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
@@ -1274,7 +1274,7 @@ static int fluid_adv_impl(const gem_cfg* cfg, const gem_grid* g, double* fluidva
   step_launch(k_ghost_epilogue<false>, grid_for(ghost_cells(g->dev.d), 256), 256, 0, st, g->dev, B);
   GEM_LAUNCHED("k_ghost_epilogue");
   if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
-    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * LSP;
+    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * 32;
     step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * g->dev.d.ng);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
@@ -1333,7 +1333,7 @@ static int advection_keepre(const gem_grid* g, double* fluidvars, double* fluida
   step_launch(k_ghost_epilogue<true>, grid_for(ghost_cells(d), 256), 256, 0, st, g->dev, B);
   GEM_LAUNCHED("k_ghost_epilogue");
   if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
-    const long long n = (long long)d.lx2 * d.lx3 * LSP;
+    const long long n = (long long)d.lx2 * d.lx3 * 32;
     step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * d.ng);
     GEM_LAUNCHED("k_clean_vel_edges");
   }
