@@ -47,7 +47,7 @@ class DiffProblem:
         self._sa = None  # gem_step_adjoint workspaces (the backward's replay slots), made on first use
         self._side = None  # the replay stream of the pipelined backward
         self.replay_slots = True  # recompute by replay + finish when k+1 workspaces fit
-        self._dtt = None
+        self._dtt = self._dtt_of = None  # the schedule on the device, and as it was copied
         self._capturing = False
         self._graphs = {}  # (Ttop given) -> captured step VJP
         self.vjp_graph = True
@@ -101,12 +101,13 @@ class DiffProblem:
                 self.v1i[..., 0].clone(), self.v1i[..., -1].clone())
 
     def dt_tensor(self, j: int):
-        """The step's dt as a cached 1-element device tensor.  The schedule is copied once, by
-        a copy the host waits for, so that any stream may read it afterwards."""
+        """The step's dt as a cached 1-element device tensor.  The schedule is copied when it
+        has changed, by a copy the host waits for, so that any stream may read it afterwards."""
         import torch
 
-        if self._dtt is None:
+        if self._dtt_of != self.dts:
             self._dtt = torch.tensor(self.dts, dtype=torch.float64, device=self.base.device)
+            self._dtt_of = list(self.dts)
         return self._dtt[j:j + 1]
 
     def cuda_step(self, j: int) -> None:
