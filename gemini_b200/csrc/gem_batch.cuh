@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(224, 2) kb_sweep_march(const InstDev* __restri
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     const Item q = it[w];
     const InstDev& I = inst[q.x];
-    b_sweep_march<DIM, UNIT, true, PERM, false, INV>(I.sw, VB{q.y, q.z, q.w});
+    if (DIM == 2 && I.sw.G.d.lx2 == 1) b_x2_single<false>(I.sw, VB{q.y, q.z, q.w});
+    else b_sweep_march<DIM, UNIT, true, PERM, false, INV>(I.sw, VB{q.y, q.z, q.w});
     if (DIM == 2) __syncthreads();  // the epilogue's shared buffers are reused by the next item
   }
 }

@@ -244,7 +244,9 @@ int launch_sweep_t(const gem_grid* g, SweepArgs a, int nsp, cudaStream_t st) {
     GEM_LAUNCHED("k_sweep_march");
     return GEM_OK;
   }
-  if (g->dev.unit)
+  if (FUSED && DIM == 2 && d.lx2 == 1)
+    step_launch(k_x2_single<false>, grid, block, 0, st, a);
+  else if (g->dev.unit)
     step_launch(k_sweep_march<DIM == 3 ? 3 : 2, true, FUSED>, grid, block, 0, st, a);
   else
     step_launch(k_sweep_march<DIM == 3 ? 3 : 2, false, FUSED>, grid, block, 0, st, a);
@@ -1325,7 +1327,9 @@ static int advection_keepre(const gem_grid* g, double* fluidvars, double* fluida
   if ((rc = launch_sweep(g, 3, true, a, LSP, st))) return rc;
   if ((rc = launch_sweep(g, 1, true, a, LSP, st))) return rc;
   const dim3 block(32, LSP), grid((d.lx1 + 31) / 32, d.lx3, a.nsB ? sweep_parts(d, 2) : 1);
-  if (g->dev.unit)
+  if (d.lx2 == 1)
+    step_launch(k_x2_single<true>, grid, block, 0, st, a);
+  else if (g->dev.unit)
     step_launch(k_sweep_march<2, true, true, 2, true>, grid, block, 0, st, a);
   else
     step_launch(k_sweep_march<2, false, true, 2, true>, grid, block, 0, st, a);

@@ -1039,7 +1039,7 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb, i
 
   if (lx <= 1) {
     // advec1D_MC_curv passes a single-cell line through; the fused x3 sweep still
-    // materialises the converted momentum/energy densities
+    // materialises the converted momentum/energy densities (fused x2: b_x2_single)
     if (FUSED && DIM == 3 && valid) {
       const unsigned k = off(1);
       if (P.nsB && ion) dst[0][k] = src[0][k];
@@ -1339,6 +1339,61 @@ __device__ __forceinline__ void b_sweep_march(const SweepArgs& P, const VB vb, i
   // nothing in flight when the next work item (batched path) restages
   cp_async_wait<0>();
   __syncwarp();
+}
+
+// The fused x2 sweep of a grid one cell wide along x2: advec1D_MC_curv passes the line through,
+// and the epilogue of the march follows on the values as they stand (where the sweeps run out
+// of place, those the x1 sweep left in the separate blocks).  A function of its own: with the
+// epilogue called from a second place the march lost registers (384x192x192 step 14.47 -> 14.87
+// ms).  Whole blocks of (32, LSP) threads call it.
+template <bool KEEPRE>
+__device__ __noinline__ void b_x2_single(const SweepArgs& P, const VB vb) {
+  const GridDev& G = P.G;
+  const Dims& d = G.d;
+  const Blocks& B = P.B;
+  const int s = threadIdx.y, lane = threadIdx.x;
+  const int a = vb.bx * 32 + lane + 1, b = vb.by + 1;
+  const bool valid = a <= d.lx1;
+  const bool ion = s < LSP - 1;
+  const long long k = gi(d, valid ? a : d.lx1, 1, b), so = s * d.ng;
+  const bool nul = valid && is_null(G, a, 1, b);
+  __shared__ double sh_n[LSP - 1][32], sh_t[LSP - 1][32];
+  const double e = (P.reB ? P.reB + so : B.re(s))[k];
+  double n = 0.0, r = 0.0, v = 0.0;
+  if (ion) {
+    n = (P.nsB ? P.nsB + so : B.ns(s))[k];
+    r = (P.rvB ? P.rvB + so : B.rv(s))[k];
+    v = r / (c_ms[s] * fmax_f(n, MINDENSDIV));
+    sh_n[s][lane] = n;
+    sh_t[s][lane] = n * c_qs[s] * v;
+    n = fmax_f(n, MINDENS);
+  }
+  __syncthreads();
+  if (!ion) {
+    double npre = 0.0, chrg = 0.0;
+    for (int q = 0; q < LSP - 1; ++q) {
+      npre = npre + sh_n[q][lane];
+      chrg = chrg + sh_t[q][lane];
+      n = n + fmax_f(sh_n[q][lane], MINDENS);
+    }
+    v = -1 / fmax_f(npre, MINDENSDIV) / QE * chrg;
+  }
+  if (nul) n = (s == 0) ? MINDENSNULL * 1e-2 : MINDENSNULL;
+  if (!valid) return;
+  B.ns(s)[k] = n;
+  B.vs1(s)[k] = nul ? 0.0 : v;
+  if (ion) B.rv(s)[k] = r;
+  if (KEEPRE) {
+    B.re(s)[k] = e;
+  } else {
+    const double T = fmax_f(c_gm1kb[s] * e / fmax_f(n, MINDENSDIV), 100.0);
+    B.Ts(s)[k] = nul ? 100.0 : T;
+  }
+}
+template <bool KEEPRE>
+__global__ void __launch_bounds__(32 * LSP) k_x2_single(SweepArgs P) {
+  step_entry();
+  b_x2_single<KEEPRE>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
 
 #ifndef GEM_MARCH_MINB
