@@ -348,8 +348,8 @@ __global__ void ka_copy_vjp(GridDev G, double* C) {
 }
 
 // Before a sweep adjoint writes the cotangent stage Cn from C: the cells its lines do not
-// cover -- the ghost frame of the other two directions, and the species past a field's
-// nsp -- keep C's value.
+// cover -- the ghost frame of the other two directions, the species past a field's nsp, and
+// single-cell lines, which the sweep passes through -- keep C's value.
 template <int DIM>
 __global__ void ka_frame_copy(GridDev G, const double* __restrict__ C, double* Cn) {
   step_entry();
@@ -367,7 +367,7 @@ __global__ void ka_frame_copy(GridDev G, const double* __restrict__ C, double* C
     const bool in2 = i2 >= 1 && i2 <= d.lx2, in3 = i3 >= 1 && i3 <= d.lx3;
     const bool swept = s < ((fld == 2) ? LSP : LSP - 1);
     // rows whose every cell some line covers (x1 lines), or whose interior x1 cells lines cover
-    const bool row_line = (DIM == 1) ? (in2 && in3) : (DIM == 2) ? in3 : in2;
+    const bool row_line = (DIM == 1) ? (in2 && in3) : (DIM == 2) ? (in3 && d.lx2 > 1) : (in2 && d.lx3 > 1);
     if (swept && row_line && DIM == 1) continue;
     const long long k0 = (long long)b * ng + gi(d, 0, i2, i3);
     for (int i1 = lane - 1; i1 <= d.lx1 + 2; i1 += 32) {
