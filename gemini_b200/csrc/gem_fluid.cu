@@ -918,6 +918,11 @@ int gem_work_prepare(gem_work* w, const gem_grid* g) {
   return work_scratch(w, g);
 }
 
+int gem_diffusion_columns(const gem_grid* g) {
+  if (check_grid(g)) return -1;
+  return luc_columns(g->dev.d);
+}
+
 int gem_work_substep_buffers(gem_work* w, const gem_source_inputs** src, double** Q, double** Pr, double** Lo) {
   if (!w) return set_err(GEM_EINVAL, "null work object");
   int rc = work_sub_alloc(w);

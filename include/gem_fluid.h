@@ -77,6 +77,10 @@ int gem_grid_dims(const gem_grid* g, int* lx1, int* lx2, int* lx3);
 int gem_work_create(const gem_grid* g, gem_work** out);
 /* allocate the work object's scratch now (before measuring free memory or capturing) */
 int gem_work_prepare(gem_work* w, const gem_grid* g);
+/* the form of the energy diffusion that a grid's sizes choose: columns per block where whole
+ * columns wait in shared memory (few columns), 0 where warps of 32 columns go through the
+ * work object's scratch, -1 for a null grid */
+int gem_diffusion_columns(const gem_grid* g);
 int gem_work_destroy(gem_work* w);
 /* copy neutral inputs (host pointers; nn (lx1,lx2,lx3,3), Tn (lx1,lx2,lx3)) */
 int gem_work_set_neutrals(gem_work* w, const double* nn, const double* Tn);
