@@ -75,11 +75,11 @@ __device__ __forceinline__ bool exp_in(double x, int lo, int hi) {
 
 // FastQ's condition for the exchange rates, with margin: densities in [2^-350, 2^200) (the
 // floor is 1e-100), temperatures in [2^-20, 2^100), neutral densities 0 or in [2^-300, 2^200),
-// and of each pair Psi in [2^-250, 1] and Phi 0 or in [2^-100, 2^100).  Then P is in
+// the neutral temperature finite (a collision frequency then stays below 2^740), and of each pair Psi in [2^-250, 1] and Phi 0 or in [2^-100, 2^100).  Then P is in
 // [2^-30, 2^150), nu at least 2^-550, the numerators at least 2^-900 and their quotients by
 // masses (2^-101 .. 2^-82) and by 3 above 2^-960: nothing leaves the normal range.  Each warp
-// tests its species, its pairs and (warps 0..3) one neutral; the block takes the fast body
-// only if all pass.
+// tests its species, its pairs and (warps 0..4) one neutral or the neutral temperature; the
+// block takes the fast body only if all pass.
 __device__ __forceinline__ bool state_ok(double n, double T) { return exp_in(n, -350, 200) && exp_in(T, -20, 100); }
 __device__ __forceinline__ bool pair_ok(const gemr::CoulPair& q) {
   return exp_in(q.Psi, -250, 1) && (exp_in(q.Phi, -100, 100) || q.Phi == 0.0);
@@ -108,9 +108,9 @@ __device__ __forceinline__ bool fill_pairs(const gemr::View& v, int isp, int lan
 // Loads the block's cells (the warp of species isp its own), then fills the pair table; true
 // when the fast bodies apply to the whole block.  The pairs' own quotients by masses need
 // only the temperatures' range.
-__device__ __forceinline__ bool load_cells(const gemr::View& v, const double* __restrict__ nn, int isp, int lane, bool in,
-                                           long long c, long long k, const double* __restrict__ fv, CellTab& cells,
-                                           PairTab& tab) {
+__device__ __forceinline__ bool load_cells(const gemr::View& v, const double* __restrict__ nn,
+                                           const double* __restrict__ Tn, int isp, int lane, bool in, long long c,
+                                           long long k, const double* __restrict__ fv, CellTab& cells, PairTab& tab) {
   bool ok = true;
   if (in) {
     double x[5];
@@ -123,6 +123,8 @@ __device__ __forceinline__ bool load_cells(const gemr::View& v, const double* __
     if (isp < gemr::NNEU) {
       const double q = nn[isp * gemr::ncell(v) + c];
       ok = ok && (exp_in(q, -300, 200) || q == 0.0);
+    } else if (isp == gemr::NNEU) {
+      ok = ok && isfinite(Tn[c]);
     }
   }
   ok = __syncthreads_and(ok);
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(kRateThreads, 5) kr_energy(gemr::View v, RateI
     gemr::cell_of(v, c, i1, i2, i3);
     k = gemr::gix(v, i1, i2, i3);
   }
-  const bool fast = load_cells(v, in.nn, isp, lane, c < nc, c, k, fv, cells, tab);
+  const bool fast = load_cells(v, in.nn, in.Tn, isp, lane, c < nc, c, k, fv, cells, tab);
   if (c >= nc) return;
   const SmemFields F{&cells, lane};
   const SmemPairs pairs{&tab, lane};
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(kRateThreads, 5) kr_momentum(gemr::View v, Rat
     gemr::cell_of(v, c, i1, i2, i3);
     kg = gemr::gix(v, i1, i2, i3);
   }
-  const bool fast = load_cells(v, in.nn, isp, lane, ok, c, kg, fv, cells, tab);
+  const bool fast = load_cells(v, in.nn, in.Tn, isp, lane, ok, c, kg, fv, cells, tab);
   const SmemFields F{&cells, lane};
   const double l0 = ok ? log(F.n(isp) * gemr::KB_ * F.T(isp)) : 0.0;
   double lm = __shfl_up_sync(0xffffffffu, l0, 1), lp = __shfl_down_sync(0xffffffffu, l0, 1);
