@@ -101,13 +101,20 @@ class DiffProblem:
                 self.v1i[..., 0].clone(), self.v1i[..., -1].clone())
 
     def dt_tensor(self, j: int):
-        """The step's dt as a cached 1-element device tensor.  The schedule is copied when it
-        has changed, by a copy the host waits for, so that any stream may read it afterwards."""
+        """The step's dt as a 1-element device tensor: a view of the schedule's device copy, which
+        is made again when the schedule has changed, by a copy the host waits for, so that any
+        stream may read it afterwards.  While the current stream is being captured, a tensor of
+        its own: the graph keeps the step it was captured with and no address of the copy."""
         import torch
 
-        if self._dtt_of != self.dts:
-            self._dtt = torch.tensor(self.dts, dtype=torch.float64, device=self.base.device)
-            self._dtt_of = list(self.dts)
+        if self.base.is_cuda and torch.cuda.is_current_stream_capturing():
+            return torch.full((1,), float(self.dts[j]), dtype=torch.float64, device=self.base.device)
+        dts = [float(x) for x in self.dts]  # a list, tuple or array
+        if self._dtt_of != dts:
+            if self._dtt is not None and self.base.is_cuda:
+                torch.cuda.synchronize()  # a pass on another stream may still read the old copy
+            self._dtt = torch.tensor(dts, dtype=torch.float64, device=self.base.device)
+            self._dtt_of = dts
         return self._dtt[j:j + 1]
 
     def cuda_step(self, j: int) -> None:
