@@ -195,14 +195,15 @@ int sweep_parts(const Dims& d, int dim) {
 
 int work_scratch(gem_work* w, const gem_grid* g);
 
-// The out-of-place blocks of the fused sweeps where a line is cut (else null): densities,
-// momentum and energy densities of all species.
+// The out-of-place blocks of the fused sweeps where a line is cut (else null, and null where
+// there was no room for them): densities, momentum and energy densities of all species.
 bool sweeps_cut(const Dims& d) { return sweep_parts(d, 2) > 1 || sweep_parts(d, 3) > 1; }
 int work_sweeps(gem_work* w, const gem_grid* g, SweepArgs& a) {
   const Dims& d = g->dev.d;
   if (!sweeps_cut(d)) return GEM_OK;
   const int rc = work_scratch(w, g);
   if (rc) return rc;
+  if (!w->sweep) return GEM_OK;
   a.nsB = w->sweep;
   a.rvB = a.nsB + LSP * d.ng;
   a.reB = a.rvB + LSP * d.ng;
@@ -356,17 +357,25 @@ int luc_columns(const Dims& d) {
 // The work object's scratch, one allocation by the first launch that needs any of it (two
 // would cost a small grid's first step 0.3 ms more): the diffusion's, the factors of every
 // column for k_diffusion_col or a slot per resident warp for k_diffusion_lu, then the cut
-// sweeps' blocks.  The batched step has its own; a work object only ever batched needs none.
+// sweeps' blocks (21 ghosted blocks, three fifths of fluidvars).  Without room for those the
+// diffusion's alone, and the sweeps run in place.  The batched step has its own; a work object
+// only ever batched needs none.
 int work_scratch(gem_work* w, const gem_grid* g) {
   if (w->lu) return GEM_OK;
   const Dims& d = g->dev.d;
   const long long lu = luc_columns(d) > 0 ? 3LL * LSP * nci(d) : lu_slots_for(d) * lu_slot_doubles(d.lx1);
-  const size_t bytes = sizeof(double) * (size_t)(lu + (sweeps_cut(d) ? 3LL * LSP * d.ng : 0));
+  const long long sweep = sweeps_cut(d) ? 3LL * LSP * d.ng : 0;
+  if (sweep && cudaMalloc(&w->lu, sizeof(double) * (size_t)(lu + sweep)) == cudaSuccess) {
+    w->sweep = w->lu + lu;
+    return GEM_OK;
+  }
+  const size_t bytes = sizeof(double) * (size_t)lu;
+  cudaGetLastError();  // of the larger request
   if (cudaMalloc(&w->lu, bytes) != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next launch's check
     w->lu = nullptr;
     return set_err(GEM_ENOMEM, "cudaMalloc of %zu bytes for the step's scratch failed", bytes);
   }
-  w->sweep = w->lu + lu;
   return GEM_OK;
 }
 
