@@ -186,14 +186,14 @@ struct gem_batch {
   cudaGraph_t graph_fixed = nullptr;  // the step with prescribed time steps
   cudaGraphExec_t exec_fixed = nullptr;
   double* d_dt_in = nullptr;  // per-instance prescribed dt (device)
-  // band-solve scratch of the instances' diffusion items, one per metric variant that has any
+  // band-solve scratch of the instances' diffusion items: the two chains' own, or one for both
   double *d_lu[2] = {nullptr, nullptr}, *lu_base[2] = {nullptr, nullptr};
   // the two variants' instances share nothing, so their launches run as two chains: where one
   // chain's phase thins out, the other's blocks fill the device (eight instances 14.7 -> 13.15 ms)
   bool variant[2] = {false, false}, two = false;
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
-  long long lu_slot = 0;      // doubles per scratch slot (the longest column's)
+  long long lu_slot[2] = {0, 0};  // doubles per scratch slot (the variant's longest column)
   int use_graph = 1;
 };
 
@@ -358,8 +358,8 @@ int batch_chain(gem_batch* b, int unit, cudaStream_t st, bool fixed_dt) {
       case BK_EPI: kb_ghost_epilogue<<<L.grid, 256, 0, st>>>(I, L.d_items, n); break;
       case BK_CVE: kb_clean_vel_edges<<<L.grid, 128, 0, st>>>(I, L.d_items, n); break;
       case BK_DIFF:
-        if (u) kb_diffusion_lu<true><<<L.grid, 32 * LU_WPB, 0, st>>>(I, L.d_items, n, b->d_lu[L.unit], b->lu_slot);
-        else kb_diffusion_lu<false><<<L.grid, 32 * LU_WPB, 0, st>>>(I, L.d_items, n, b->d_lu[L.unit], b->lu_slot);
+        if (u) kb_diffusion_lu<true><<<L.grid, 32 * LU_WPB, 0, st>>>(I, L.d_items, n, b->d_lu[L.unit], b->lu_slot[L.unit]);
+        else kb_diffusion_lu<false><<<L.grid, 32 * LU_WPB, 0, st>>>(I, L.d_items, n, b->d_lu[L.unit], b->lu_slot[L.unit]);
         break;
     }
   }
@@ -402,21 +402,31 @@ int gem_batch_create(int n, const gem_grid* const* grids, gem_work* const* works
   std::vector<InstDev> h(n);
   gem_batch* b = new gem_batch();
   b->n = n;
-  int lx1_max = 0;
+  // per variant, a scratch slot for every warp of its diffusion launch (launch_grid)
+  int lx1_max[2] = {0, 0};
+  long long nblk[2] = {0, 0};
   for (int i = 0; i < n; ++i)
-    if (grids[i]) lx1_max = std::max(lx1_max, grids[i]->dev.d.lx1);
-  b->lu_slot = lu_slot_doubles(lx1_max);
-  for (int i = 0; i < n; ++i)
-    if (grids[i]) b->variant[grids[i]->dev.unit ? 1 : 0] = true;
-  const size_t lu_bytes = sizeof(double) * lu_slots() * b->lu_slot;
-  if (cudaMalloc(&b->lu_base[0], lu_bytes) != cudaSuccess) {
+    if (grids[i]) {
+      const int u = grids[i]->dev.unit ? 1 : 0;
+      b->variant[u] = true;
+      lx1_max[u] = std::max(lx1_max[u], grids[i]->dev.d.lx1);
+      nblk[u] += lu_tasks(grids[i]->dev.d) / LU_WPB;
+    }
+  size_t need[2];
+  for (int u = 0; u < 2; ++u) {
+    b->lu_slot[u] = lu_slot_doubles(lx1_max[u]);
+    need[u] = sizeof(double) * std::min(nblk[u] * LU_WPB, lu_slots()) * b->lu_slot[u];
+  }
+  const int big = need[1] > need[0] ? 1 : 0;
+  if (need[big] && cudaMalloc(&b->lu_base[0], need[big]) != cudaSuccess) {
+    cudaGetLastError();
     delete b;
-    return set_err(GEM_ENOMEM, "cudaMalloc of the batch's band-solve scratch failed");
+    return set_err(GEM_ENOMEM, "cudaMalloc of %zu bytes for the batch's band-solve scratch failed", need[big]);
   }
   b->d_lu[0] = b->d_lu[1] = b->lu_base[0];
   if (b->variant[0] && b->variant[1]) {  // two chains need a scratch each; without room, one chain
-    b->two = cudaMalloc(&b->lu_base[1], lu_bytes) == cudaSuccess;
-    if (b->two) b->d_lu[1] = b->lu_base[1];
+    b->two = cudaMalloc(&b->lu_base[1], need[1 - big]) == cudaSuccess;
+    if (b->two) b->d_lu[1 - big] = b->lu_base[1];
     else cudaGetLastError();
   }
   for (int i = 0; i < n; ++i) {
@@ -458,7 +468,7 @@ int gem_batch_create(int n, const gem_grid* const* grids, gem_work* const* works
     I.df.Teinf = cfgs[i].Teinf;
     I.df.Ttop = w->Ttop;
     I.df.lu = b->d_lu[I.sw.G.unit ? 1 : 0];
-    I.df.lu_slot = b->lu_slot;
+    I.df.lu_slot = b->lu_slot[I.sw.G.unit ? 1 : 0];
     I.df.x3fast = (!g->dev.unit && g->dev.c3 == 0) ? 1 : 0;
     I.df.solver = cfgs[i].diffsolvetype;
     I.df.fused = 1;

@@ -69,11 +69,13 @@ int gem_grid_create(const gem_grid_desc* desc, gem_grid** out);
 int gem_grid_destroy(gem_grid* g);
 int gem_grid_dims(const gem_grid* g, int* lx1, int* lx2, int* lx3);
 /* The work object holds the per-grid state of the step (interface velocities, neutral inputs,
- * dt, reductions).  The step's scratch (for the diffusion a slot of lx1 + 4 rows per resident
- * warp, 0.5 GB for 384-row columns; on grids with few lines also blocks for the sweeps) is
- * allocated by the first gem_energy_diffusion_dev / gem_fluid_adv_dev call that uses the work
- * object: make that first call before capturing these calls in a CUDA graph.  Work objects
- * that only take part in a gem_batch never allocate it (the batch has its own). */
+ * dt, reductions).  The step's scratch is allocated by the first gem_energy_diffusion_dev /
+ * gem_fluid_adv_dev call that uses the work object: make that first call before capturing
+ * these calls in a CUDA graph.  It holds the diffusion's part (on grids with few columns 21
+ * doubles a cell; else a slot of 4.75 doubles a row and lane per resident warp, 1.1 GB for
+ * 384-row columns on 148 SMs) and, on grids with few lines along x2 or x3, 21 ghosted blocks for
+ * the sweeps (three fifths of fluidvars), which are left out where they do not fit.  Work
+ * objects that only take part in a gem_batch never allocate it (the batch has its own). */
 int gem_work_create(const gem_grid* g, gem_work** out);
 /* allocate the work object's scratch now (before measuring free memory or capturing) */
 int gem_work_prepare(gem_work* w, const gem_grid* g);
@@ -363,7 +365,10 @@ int gem_dt_calc_noalloc_dev(const gem_grid* g, double tcfl, const double* fluidv
  * step's launches are captured once into a CUDA graph that later calls replay (on any
  * stream).  Each instance's dt is computed into its work object's dt slot (gem_work_dt).
  * The batch keeps pointers to the objects it was given: they must outlive it and must not
- * move.  Tuning parameters (gem_batch_set_param) rebuild the work lists and the graph. */
+ * move.  Tuning parameters (gem_batch_set_param) rebuild the work lists and the graph.
+ * The batch holds a diffusion scratch: a slot for every resident warp that its instances' columns
+ * can fill (up to 1.1 GB for 384-row columns), and a second one where instances with unit and
+ * with tabulated metrics are mixed, which then run as two chains (without room, as one). */
 typedef struct gem_batch gem_batch;
 #define GEM_BATCH_USE_GRAPH 0  /* 1 (default): capture the step into a CUDA graph */
 #define GEM_BATCH_DIFF_BLOCKS 1 /* resident diffusion blocks (4 warps each) per SM, 1..4 (default 4) */

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from gemini_b200 import _lib
+from gemini_b200 import batch as BT
 from gemini_b200 import fluid as F
 from gemini_b200 import grid as G
 from gemini_b200 import workloads as WL
@@ -56,3 +57,57 @@ def test_step_without_room_for_cut_lines(compression):
     b.close()
     for x, y in zip(got, want):
         assert torch.equal(x, y)
+
+
+def _mixed(lx1, lx23, n):
+    """n Cartesian and n dipole instances of the same sizes, and their plain copies."""
+    grids = [G.cartesian_grid(lx1, lx23, lx23) for _ in range(n)] + [G.dipole_grid(lx1, lx23, lx23) for _ in range(n)]
+    out = []
+    for k, g in enumerate(grids):
+        dg = F.DeviceGrid(g)
+        a, b = (WL.device_state(dg, g, k) for _ in range(2))
+        b.fluidvars.copy_(a.fluidvars)
+        b.fluidauxvars.copy_(a.fluidauxvars)
+        out.append(((dg, a, F.FluidCfg(a.Teinf)), (dg, b, F.FluidCfg(b.Teinf))))
+    return out
+
+
+def _batch_bytes(insts):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    b = BT.Batch(insts)
+    return b, before - torch.cuda.mem_get_info()[0]
+
+
+def _check(b, insts):
+    for _ in range(2):
+        b.step()
+        for _, p in insts:
+            BT.plain_step(*p)
+    torch.cuda.synchronize()
+    for (_, x, _), (_, y, _) in insts:
+        assert torch.equal(x.fluidvars, y.fluidvars) and torch.equal(x.fluidauxvars, y.fluidauxvars)
+
+
+def test_batch_scratch_fits_its_instances():
+    """Two instances of 40x8x8 are 14 warps of columns each: a few MB, not a slot for every warp
+    that the device holds."""
+    insts = _mixed(40, 8, 1)
+    BT.Batch([i[0] for i in insts]).close()  # loads the kernels
+    b, used = _batch_bytes([i[0] for i in insts])
+    assert used < 16 * MB, used
+    _check(b, insts)
+
+
+def test_batch_without_room_for_two_chains():
+    """Mixed instances that fill every slot of both variants: with room for one scratch only, the
+    batch runs as one chain, with the same bits."""
+    insts = _mixed(200, 80, 2)
+    first = [i[0] for i in insts]
+    b, both = _batch_bytes(first)
+    b.close()
+    with _left(both - both // 4):
+        b, one = _batch_bytes(first)
+    assert one < both - both // 4
+    _check(b, insts)
