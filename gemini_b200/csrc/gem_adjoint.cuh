@@ -744,10 +744,7 @@ int gem_step_vjp_finish_dev(const gem_cfg* cfg, const gem_grid* g, gem_work* w, 
   GEM_LAUNCHED("ka_finish_fwd");
   step_launch(k_ghost_epilogue<false>, grid_for(ghost_cells(d), 256), 256, 0, st, G, B);
   GEM_LAUNCHED("k_ghost_epilogue");
-  if (G.has_null && (G.gridflag == 0 || G.gridflag == 1)) {
-    step_launch(k_clean_vel_edges, grid_for(ncol * LSP, 128), 128, 0, st, G, fluidvars + LSP * d.ng);
-    GEM_LAUNCHED("k_clean_vel_edges");
-  }
+  if ((rc = launch_clean_vel_edges(g, fluidvars + LSP * d.ng, st))) return rc;
   DiffArgs da;
   da.G = G;
   da.B = B;

@@ -290,8 +290,7 @@ int batch_build_lists(gem_batch* b) {
           case BK_SW2: add_items(launch_for(k, u), i, gx13, d.lx3); break;
           case BK_EPI: add_items(launch_for(k, u), i, grid_for(ghost_cells(d), 256)); break;
           case BK_CVE:
-            if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1))
-              add_items(launch_for(k, u), i, grid_for((long long)d.lx2 * d.lx3 * LSP, 128));
+            if (has_vel_edges(g->dev)) add_items(launch_for(k, u), i, clean_vel_blocks(d));
             break;
           case BK_DIFF: {
             const long long ntask = (((long long)d.lx2 * d.lx3 + 31) / 32) * LSP;

@@ -103,6 +103,9 @@ unsigned dt_blocks(const Dims& d) {
   return (unsigned)std::min<long long>((long long)d.lx2 * d.lx3, (long long)num_sms() * 4);
 }
 
+// blocks of 128 threads for the null-edge velocity fix, a warp per column
+unsigned clean_vel_blocks(const Dims& d) { return grid_for((long long)d.lx2 * d.lx3 * 32, 128); }
+
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 }  // namespace
@@ -207,6 +210,15 @@ int work_sweeps(gem_work* w, const gem_grid* g, SweepArgs& a) {
   a.nsB = w->sweep;
   a.rvB = a.nsB + LSP * d.ng;
   a.reB = a.rvB + LSP * d.ng;
+  return GEM_OK;
+}
+
+// clean_param(2)'s border fix, where a grid has null cells and that type (multifluid.f90:614-654)
+bool has_vel_edges(const GridDev& G) { return G.has_null && (G.gridflag == 0 || G.gridflag == 1); }
+int launch_clean_vel_edges(const gem_grid* g, double* vs1, cudaStream_t st) {
+  if (!has_vel_edges(g->dev)) return GEM_OK;
+  step_launch(k_clean_vel_edges, clean_vel_blocks(g->dev.d), 128, 0, st, g->dev, vs1);
+  GEM_LAUNCHED("k_clean_vel_edges");
   return GEM_OK;
 }
 
@@ -1068,24 +1080,14 @@ int gem_clean_param_dev(const gem_grid* g, int iparm, double* fluidvars, void* s
   double* param = fluidvars + (iparm == 1 ? 0 : iparm == 2 ? LSP : 4 * LSP) * ng;
   step_launch(k_clean_elementwise, grid_for(ng, 256), 256, 0, S(stream), g->dev, param, iparm);
   GEM_LAUNCHED("k_clean_elementwise");
-  if (iparm == 2 && g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
-    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * 32;
-    step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, S(stream), g->dev, param);
-    GEM_LAUNCHED("k_clean_vel_edges");
-  }
-  return GEM_OK;
+  return iparm == 2 ? launch_clean_vel_edges(g, param, S(stream)) : GEM_OK;
 }
 
 // clean_param(3), (2), (1) in the order the source sub-step ends with
 static int clean_all(const gem_grid* g, double* fluidvars, cudaStream_t st) {
   step_launch(k_clean_all, grid_for(g->dev.d.ng, 256), 256, 0, st, g->dev, blocks(g, fluidvars, nullptr));
   GEM_LAUNCHED("k_clean_all");
-  if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
-    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * 32;
-    step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * g->dev.d.ng);
-    GEM_LAUNCHED("k_clean_vel_edges");
-  }
-  return GEM_OK;
+  return launch_clean_vel_edges(g, fluidvars + LSP * g->dev.d.ng, st);
 }
 
 int gem_energy_diffusion_dev(const gem_cfg* cfg, const gem_grid* g, double* fluidvars,
@@ -1289,11 +1291,7 @@ static int fluid_adv_impl(const gem_cfg* cfg, const gem_grid* g, double* fluidva
   w->timer.record(5, st);
   step_launch(k_ghost_epilogue<false>, grid_for(ghost_cells(g->dev.d), 256), 256, 0, st, g->dev, B);
   GEM_LAUNCHED("k_ghost_epilogue");
-  if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
-    const long long n = (long long)g->dev.d.lx2 * g->dev.d.lx3 * 32;
-    step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * g->dev.d.ng);
-    GEM_LAUNCHED("k_clean_vel_edges");
-  }
+  if ((rc = launch_clean_vel_edges(g, fluidvars + LSP * g->dev.d.ng, st))) return rc;
   if (after_epi) GEM_CUDA(cudaEventRecord(after_epi, st));
   DiffArgs d;
   d.G = g->dev;
@@ -1350,12 +1348,7 @@ static int advection_keepre(const gem_grid* g, double* fluidvars, double* fluida
   GEM_LAUNCHED("k_sweep_march");
   step_launch(k_ghost_epilogue<true>, grid_for(ghost_cells(d), 256), 256, 0, st, g->dev, B);
   GEM_LAUNCHED("k_ghost_epilogue");
-  if (g->dev.has_null && (g->dev.gridflag == 0 || g->dev.gridflag == 1)) {
-    const long long n = (long long)d.lx2 * d.lx3 * 32;
-    step_launch(k_clean_vel_edges, grid_for(n, 128), 128, 0, st, g->dev, fluidvars + LSP * d.ng);
-    GEM_LAUNCHED("k_clean_vel_edges");
-  }
-  return GEM_OK;
+  return launch_clean_vel_edges(g, fluidvars + LSP * d.ng, st);
 }
 
 // energy_diffusion, clean_param(3) and T2rhoe of the step with compression: the diffusion's

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import oracle as O
+from gemini_b200 import batch as BT
 from gemini_b200 import fluid as F
 from gemini_b200 import grid as G
 from gemini_b200 import state as S
@@ -32,3 +33,18 @@ def test_null_edges(lx1, gridflag):
     O.clean_param(g, st, 2)
     F.clean_param(ds, 2)
     assert_identical(ds.to_host(st), st, "clean_param(2)")
+
+
+def test_batched_work_items():
+    """The batched fix gets a warp per column too: four columns per work item of 128 threads."""
+    g = G.dipole_grid(40, 9, 7, q_extent=0.5)
+    assert g.nullpts.any()
+    items = []
+    for nulls in (True, False):
+        g.nullpts = g.nullpts & nulls
+        st = S.init_state(g, seed=1)
+        dg = F.DeviceGrid(g)
+        b = BT.Batch([(dg, F.DeviceState.from_host(dg, st), F.FluidCfg(st.Teinf))])
+        items.append(b.info()[1])
+        b.close()
+    assert items[0] - items[1] == (9 * 7 + 3) // 4
