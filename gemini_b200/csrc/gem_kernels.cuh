@@ -1610,8 +1610,11 @@ __device__ __forceinline__ void b_sweep_x1(const SweepArgs& P, const VB vb) {
   cp_async_wait<0>();  // nothing in flight when the next work item (batched path) restages
 }
 
+// Blocks per SM: three fields need the registers of three (fused) or two (and out of place); a
+// single field on unit metrics runs at five with 56 registers (384x192x192, six species 875 -> 824
+// us, at three 892; seven species 1064 -> 968), on tabulated ones five spill (1630 against 1211).
 template <bool UNIT, bool FUSED, bool OOP = false>
-__global__ void __launch_bounds__(224, OOP ? 2 : 3) k_sweep_x1(SweepArgs P) {
+__global__ void __launch_bounds__(224, OOP ? 2 : !FUSED && UNIT ? 5 : 3) k_sweep_x1(SweepArgs P) {
   step_entry();
   b_sweep_x1<UNIT, FUSED, OOP>(P, VB{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x});
 }
