@@ -97,6 +97,15 @@ void step_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cud
   cudaLaunchKernelEx(&c, kern, KArgs(args)...);
 }
 
+// Lets a kernel's launches use any dynamic shared memory a block can have.  The limit belongs to
+// the kernel, not the launch: always the same value, so that a thread which launches a smaller
+// grid's block cannot lower it between another thread's setting and launch.
+constexpr size_t MAX_SMEM = 227 * 1024;
+template <class K>
+cudaError_t allow_smem(K* kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM);
+}
+
 // blocks of the dt and CFL reductions: a block per x1 row up to the four an SM holds (eight, a
 // second partial wave: 96x32x32 20.4 us against 17.3; the same at 384x192x192)
 unsigned dt_blocks(const Dims& d) {
@@ -352,7 +361,7 @@ long long lu_slots_for(const Dims& d) { return std::min(lu_slots(), lu_tasks(d))
 // 128x64x64 470 / 288, 64x96x96 371 / 206.
 size_t luc_bytes(int lx1) { return sizeof(double) * luc_pitch(lx1); }
 int luc_columns(const Dims& d) {
-  constexpr size_t SM_BYTES = 227 * 1024, BLOCK_OVERHEAD = 1024;
+  constexpr size_t SM_BYTES = MAX_SMEM, BLOCK_OVERHEAD = 1024;
   const long long ncol = (long long)d.lx2 * d.lx3;
   const long long per_sm = (ncol * LSP + num_sms() - 1) / num_sms();  // (column, species) pairs per SM
   const long long fit = (long long)(SM_BYTES / luc_bytes(d.lx1));
@@ -408,7 +417,7 @@ int launch_diffusion_lu(const gem_grid* g, DiffArgs a, cudaStream_t st) {
     const int warps = std::min(LUC_THREADS / 32, cb * ((d.lx1 + 31) / 32));
     const size_t sm = luc_bytes(d.lx1) * cb;
     auto kern = g->dev.unit ? k_diffusion_col<true> : k_diffusion_col<false>;
-    if (sm > 48 * 1024) GEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (sm > 48 * 1024) GEM_CUDA(allow_smem(kern));
     step_launch(kern, (unsigned)(ng * LSP), 32 * warps, sm, st, a, cb);
     GEM_LAUNCHED("k_diffusion_col");
     return GEM_OK;
@@ -505,14 +514,14 @@ int launch_diffusion_vjp(const gem_grid* g, DiffAdjArgs a, cudaStream_t st) {
   const int M = std::max(2, (d.lx1 + 31) / 32);
   a.M = M;
   const size_t per_warp = (size_t)VNA * M * 32 * sizeof(double);
-  if (per_warp > 227 * 1024) return set_err(GEM_EINVAL, "lx1=%d too long for the on-chip column adjoint", d.lx1);
+  if (per_warp > MAX_SMEM) return set_err(GEM_EINVAL, "lx1=%d too long for the on-chip column adjoint", d.lx1);
   auto kern = g->dev.unit ? k_diffusion_vjp<true> : k_diffusion_vjp<false>;
+  GEM_CUDA(allow_smem(kern));
   // warps per block: the choice (4, 2 or 1) that keeps the most warps resident per SM
   int wpb = 1, best = 0, best_per_sm = 1;
   for (int w : {4, 2, 1}) {
     const size_t sm = per_warp * w;
-    if (sm > 227 * 1024) continue;
-    GEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (sm > MAX_SMEM) continue;
     int per_sm = 0;
     GEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * w, sm));
     if (per_sm * w > best) {
@@ -522,7 +531,6 @@ int launch_diffusion_vjp(const gem_grid* g, DiffAdjArgs a, cudaStream_t st) {
     }
   }
   const size_t smem = per_warp * wpb;
-  GEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long long ncs = (long long)d.lx2 * d.lx3 * LSP;
   long long nblk = (ncs + wpb - 1) / wpb;
   const long long cap = (long long)num_sms() * std::max(best_per_sm, 1);
