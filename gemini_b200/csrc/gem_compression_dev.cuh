@@ -36,8 +36,6 @@ __global__ void kc_compression(gemc::View v, long long n, const double* __restri
     gemc::cmp(v, t, vs1, vs2, vs3, Q, rhoes, dt);
 }
 
-// the View of a grid: device metric tables (null on unit-metric grids) and the species
-// constants from the same literal expressions as the device constants
 // VNRicht_artvisc, compression, rhoe2T and clean_param(3) of the interior cells in one pass:
 // Q and the new temperature of one cell and species (blockIdx.y).  The ghost velocities that
 // halo_fluidvars and RK2_global_boundary would leave are read as the interior cells they copy
@@ -113,6 +111,8 @@ __global__ void __launch_bounds__(256, 8) kc_compress_T(GridDev G, Blocks B, dou
   }
 }
 
+// the View of a grid: device metric tables (null on unit-metric grids) and the species
+// constants from the same literal expressions as the device constants
 gemc::View cmp_view(const gem_grid* g) {
   const GridDev& G = g->dev;
   const Dims& d = G.d;

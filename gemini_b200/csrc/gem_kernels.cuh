@@ -2277,7 +2277,7 @@ __device__ __forceinline__ void luc_solve(const gemd::LuK& k, double* W) {
 template <bool UNIT>
 struct LucAcc {
   const DiffArgs& P;
-  long long mofs, qofs, jofs;
+  long long mofs;  // cell 0 in the metric tables
   __device__ __forceinline__ void metrics(int i, double& a1, double& a2, double& a3, double& y1, double& ha,
                                           double& yha) const {
     const long long k = mofs + i;
@@ -2319,7 +2319,7 @@ __device__ __forceinline__ void b_diffusion_col(const DiffArgs& P, int s, int co
   };
   each([&](int, int i, int i2, int i3, double* w) {  // C, B, D of every cell
     const long long m = gi(d, i, i2, i3);
-    const LucAcc<UNIT> a{P, cmi(P.G, 0, i2, i3), 0, 0};
+    const LucAcc<UNIT> a{P, cmi(P.G, 0, i2, i3)};
     gemd::CellIn cin;
     cin.T = T[m];
     cin.n = __ldg(nv + m);
@@ -2344,7 +2344,7 @@ __device__ __forceinline__ void b_diffusion_col(const DiffArgs& P, int s, int co
     gemd::BandRow r{0.0, 1.0, 0.0, 0.0};
     if (i == 1) return;
     if (i < n) {
-      const LucAcc<UNIT> a{P, 0, 0, 0};
+      const LucAcc<UNIT> a{P, 0};
       const gemd::RowFac f = gemd::row_factors<ELEC>(a, i, w[0], w[1], w[4 - LUC_ROW], w[4], w[4 + LUC_ROW]);
       const double* Tc = T + gi(d, i, i2, i3);
       r = gemd::band_row<STG1>(t, f.qm, f.qp, f.bq, Tc[-1], Tc[0], Tc[1],
