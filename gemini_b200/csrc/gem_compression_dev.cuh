@@ -42,8 +42,8 @@ __global__ void kc_compression(gemc::View v, long long n, const double* __restri
 // (the edge cell, or the wrapped one along a periodic x3); Q reads the x1 ghosts as the
 // advection left them.  rhoes is not stored: after this only its conversion to T is used, and
 // the diffusion's store rewrites it.  Quotients through the grid's reciprocal tables (exact).
-// One pass instead of four; 384x96x96: 0.93 -> 0.47 ms at eight blocks per SM (32 registers; 0.50
-// at 48), half the copy peak by the eight doubles a cell and species needs.
+// One pass instead of four; 384x96x96: 0.93 -> 0.47 ms at eight blocks per SM (32 registers, 32-48
+// bytes spilled; 0.50 ms at 48 registers), half the copy peak by the eight doubles a cell and species needs.
 template <bool UNIT>
 __global__ void __launch_bounds__(256, 8) kc_compress_T(GridDev G, Blocks B, double* __restrict__ Q, const double* __restrict__ dtp) {
   step_entry();

@@ -13,7 +13,8 @@ struct RateIn {  // interior neutral inputs
 };
 
 // Bound by latency (a thread per cell, ten powers in a row): eight blocks per SM at 64
-// registers 0.41 ms for 384x96x96, its natural 124 registers 0.46, five or six blocks 0.56-0.59.
+// registers (204 bytes spilled) 0.41 ms for 384x96x96, its natural 124 registers 0.46, five or six
+// blocks 0.56-0.59.
 __global__ void __launch_bounds__(128, 8) kr_continuity(gemr::View v, RateIn in, const double* __restrict__ fv, double* __restrict__ Pr,
                               double* __restrict__ Lo) {
   step_entry();
@@ -184,8 +185,8 @@ struct SharedX1 {
 // are the adjacent lanes (c +- 1), except across the block's edges (lanes 0 and 31), which
 // form that one neighbour's log themselves.  At the line ends the missing side is the cell
 // itself, as the direct form's clamped neighbour index gives.
-// Five 7-warp blocks per SM (56 registers): each SM sub-partition holds a quarter of the
-// register file, so at the kernel's natural 90-odd registers only 5 warps fit per
+// Five 7-warp blocks per SM (56 registers, 420 bytes spilled, both bodies being inlined): each SM
+// sub-partition holds a quarter of the register file, so at the kernel's natural 90-odd registers only 5 warps fit per
 // sub-partition and two blocks per SM.  384x96x96: 2.08 ms, four blocks 2.28, six 2.26; before
 // the fast quotients and the shared cell table, 2.78 ms.
 __global__ void __launch_bounds__(kRateThreads, 5) kr_momentum(gemr::View v, RateIn in, const double* __restrict__ fv,
