@@ -361,9 +361,9 @@ int gem_dt_calc_noalloc_dev(const gem_grid* g, double tcfl, const double* fluidv
  * simulations, each with its own grid, work object, state blocks (device) and gem_cfg,
  * advanced together.  One gem_batch_step = gem_dt_calc_dev(cfg.tcfl) + gem_fluid_adv_dev
  * for every instance, with the same results bit for bit.  Each phase of the step is one
- * persistent launch over an (instance, block) work list, largest instances first, and the
- * step's launches are captured once into a CUDA graph that later calls replay (on any
- * stream).  Each instance's dt is computed into its work object's dt slot (gem_work_dt).
+ * launch per metric variant (unit, tabulated) over an (instance, block) work list, largest
+ * instances first, and the step's launches are captured once into a CUDA graph that later
+ * calls replay (on any stream).  Each instance's dt is computed into its work object's dt slot (gem_work_dt).
  * The batch keeps pointers to the objects it was given: they must outlive it and must not
  * move.  Tuning parameters (gem_batch_set_param) rebuild the work lists and the graph.
  * The batch holds a diffusion scratch: a slot for every resident warp that its instances' columns

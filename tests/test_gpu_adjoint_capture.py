@@ -39,3 +39,34 @@ def test_captured_step(used):
     assert torch.equal(run(graph.replay), want)
     assert torch.equal(run(lambda: P.cuda_step(0)), other)
     del hold
+
+
+@pytest.mark.parametrize("k", [1, 2])
+def test_captured_gradient(k):
+    """Forward and backward in one captured graph, replayed after the schedule has changed."""
+    g = G.cartesian_grid(24, 8, 6)
+    P = AD.DiffProblem(g, S.init_state(g, seed=2, perturb=0.1), 4, checkpoint_every=k)
+    x = P.base[(slice(0, 6), slice(2, -2), slice(2, -2), slice(2, -2))].clone().requires_grad_(True)
+
+    def grad():
+        ns, Ts = AD.FluidAdvance.apply(x, None, P)
+        return torch.autograd.grad(ns.sum() * 1e-11 + (Ts * Ts).sum() * 1e-6, [x])[0]
+
+    want = grad().clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        grad()
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = grad()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    P.dts = [0.5 * d for d in P.dts]
+    assert not torch.equal(grad(), want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
